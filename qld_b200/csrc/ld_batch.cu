@@ -262,47 +262,60 @@ k_ld_batch(const BatchParams bp) {
         }
     } else if (warp == 1) {
         // ------------------------------------------- MMA issuer (rank 0) --
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t sf = tmem + SF_COL;
-            int gu = 0, it_n = 0;
+            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UA));
+            const uint32_t b_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UB));
+            uint32_t s = 0, ph = 0;      // unpacked stage and its phase
+            int it_n = 0;
             bool ok = true;
             for (int qi = 0; ok; ++qi, ++it_n) {
                 const int slot = qi % QSLOTS;
-                if (!wait_item(qi)) {
-                    flag_error(bp.status, ST_TIMEOUT_UNPACK);
+                if (!__all_sync(0xffffffffu, wait_item(qi))) {
+                    if (lane == 0) flag_error(bp.status, ST_TIMEOUT_UNPACK);
                     break;
                 }
                 const Item it = items[slot];
                 if (it.job < 0) break;
                 const int ab = it_n & 1;
-                if (it_n >= 2 && !mbar_wait(smem_u32(&accempty[ab]), ((it_n >> 1) - 1) & 1, limit,
-                                            bp.status)) {
-                    flag_error(bp.status, ST_TIMEOUT_MMA);
-                    break;
+                if (it_n >= 2) {
+                    const bool free = mbar_wait(smem_u32(&accempty[ab]), ((it_n >> 1) - 1) & 1,
+                                                limit, bp.status);
+                    if (!__all_sync(0xffffffffu, free)) {
+                        if (lane == 0) flag_error(bp.status, ST_TIMEOUT_MMA);
+                        break;
+                    }
                 }
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)ab * ACC_STRIDE;
-                for (int u = 0; u < it.np * SUB; ++u, ++gu) {
-                    const int s = gu % UST;
-                    if (!mbar_wait(smem_u32(&ufull[s]), (gu / UST) & 1, limit, bp.status)) {
-                        flag_error(bp.status, ST_TIMEOUT_UNPACK);
+                for (int u = 0; u < it.np * SUB; ++u) {
+                    const bool full = mbar_wait(smem_u32(&ufull[s]), ph, limit, bp.status);
+                    if (!__all_sync(0xffffffffu, full)) {
+                        if (lane == 0) flag_error(bp.status, ST_TIMEOUT_UNPACK);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a0 = smem_u32(smem + L::OFF_UA + s * UA_BYTES);
-                    const uint32_t b0 = smem_u32(smem + L::OFF_UB + s * UB_BYTES);
+                    const uint32_t da = a_lo + s * (UA_BYTES >> 4), db = b_lo + s * (UB_BYTES >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        tc_mma_mxf4_pair(d, sw128_desc(a0 + kk * 32), sw128_desc(b0 + kk * 32),
-                                         (kk & 1) ? IDESC_ODD : IDESC_EVEN,
-                                         (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
-                    tc_commit_pair(smem_u32(&uempty[s]), BOTH);
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
+                                                (kk & 1) ? IDESC_ODD : IDESC_EVEN,
+                                                (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                        tc_commit_pair(smem_u32(&uempty[s]), BOTH);
+                    }
+                    __syncwarp();
+                    if (++s == UST) s = 0, ph ^= 1;
                 }
-                tc_commit_pair(smem_u32(&accfull[ab]), BOTH);
-                release_item(qi);
+                if (elect_one()) {
+                    tc_commit_pair(smem_u32(&accfull[ab]), BOTH);
+                    release_item(qi);
+                }
+                __syncwarp();
             }
-            tc_commit_pair(smem_u32(mma_done), BOTH);
+            if (elect_one()) tc_commit_pair(smem_u32(mma_done), BOTH);
+            __syncwarp();
         }
     } else if (warp < FIRST_EPI_WARP) {
         // --------------------------------------------------------- unpack --

@@ -20,7 +20,9 @@
 //   warp 1       TMEM allocation for the pair (cta_group::2); in rank 0 the
 //                MMA issuer: per unpacked stage (256 samples) 4 MMAs of
 //                256 x 240 x 64, then one commit that arrives on the stage's
-//                "empty" barrier in both CTAs.
+//                "empty" barrier in both CTAs.  The whole warp runs the issue
+//                loop (tcgen05.cuh, elect_one): single region 2.39 -> 2.375
+//                ms, band of 5,000 over 24,000 x 100,000 3.45 -> 3.39 ms.
 //   warps 2-11   unpack (w -> four words of nibbles, as ld_mxf4.cu) into the
 //                CTA's stage; they arrive on rank 0's "full" barrier.  Two
 //                groups of five warps take alternate unpacked stages (each
@@ -198,40 +200,50 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp == 1) {
         // ------------------------------------------- MMA issuer (rank 0) --
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {
             const uint32_t sf = tmem + SF_COL;
-            int gu = 0;
+            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UA));
+            const uint32_t b_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UB));
+            uint32_t s = 0, ph = 0;      // unpacked stage and its phase
             bool ok = true;
             for (int it = 0; it < my_tiles && ok; ++it) {
                 const int ab = it & 1;
-                if (it >= 2 && !mbar_wait(smem_u32(&accempty[ab]), ((it >> 1) - 1) & 1,
-                                                  p.timeout_cycles, p.status)) {
-                    flag_error(p.status, ST_TIMEOUT_MMA);
-                    break;
+                if (it >= 2) {
+                    const bool free = mbar_wait(smem_u32(&accempty[ab]), ((it >> 1) - 1) & 1,
+                                                p.timeout_cycles, p.status);
+                    if (!__all_sync(0xffffffffu, free)) {
+                        if (lane == 0) flag_error(p.status, ST_TIMEOUT_MMA);
+                        break;
+                    }
                 }
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)ab * ACC_STRIDE;
-                for (int u = 0; u < nu; ++u, ++gu) {
-                    const int s = gu % UST;
-                    if (!mbar_wait(smem_u32(&ufull[s]), (gu / UST) & 1, p.timeout_cycles,
-                                           p.status)) {
-                        flag_error(p.status, ST_TIMEOUT_UNPACK);
+                for (int u = 0; u < nu; ++u) {
+                    const bool full = mbar_wait(smem_u32(&ufull[s]), ph, p.timeout_cycles,
+                                                p.status);
+                    if (!__all_sync(0xffffffffu, full)) {
+                        if (lane == 0) flag_error(p.status, ST_TIMEOUT_UNPACK);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t a0 = smem_u32(smem + L::OFF_UA + s * UA_BYTES);
-                    const uint32_t b0 = smem_u32(smem + L::OFF_UB + s * UB_BYTES);
+                    const uint32_t da = a_lo + s * (UA_BYTES >> 4), db = b_lo + s * (UB_BYTES >> 4);
+                    if (elect_one()) {
 #pragma unroll
-                    for (int kk = 0; kk < 4; ++kk)
-                        tc_mma_mxf4_pair(d, sw128_desc(a0 + kk * 32), sw128_desc(b0 + kk * 32),
-                                         (kk & 1) ? IDESC_ODD : IDESC_EVEN,
-                                         (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
-                    tc_commit_pair(smem_u32(&uempty[s]), BOTH);
+                        for (int kk = 0; kk < 4; ++kk)
+                            tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
+                                                (kk & 1) ? IDESC_ODD : IDESC_EVEN,
+                                                (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                        tc_commit_pair(smem_u32(&uempty[s]), BOTH);
+                    }
+                    __syncwarp();
+                    if (++s == UST) s = 0, ph ^= 1;
                 }
-                tc_commit_pair(smem_u32(&accfull[ab]), BOTH);
+                if (elect_one()) tc_commit_pair(smem_u32(&accfull[ab]), BOTH);
+                __syncwarp();
             }
-            tc_commit_pair(smem_u32(mma_done), BOTH);
+            if (elect_one()) tc_commit_pair(smem_u32(mma_done), BOTH);
+            __syncwarp();
         }
     } else if (warp < FIRST_EPI_WARP) {
         // --------------------------------------------------------- unpack --

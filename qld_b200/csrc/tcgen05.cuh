@@ -107,6 +107,18 @@ __device__ __forceinline__ void tc_st_32x32b_x16_fill(uint32_t taddr, uint32_t x
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+// Write 16 consecutive TMEM columns of the warp's 32 lanes.
+__device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
+        "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]),
+        "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile(
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
@@ -202,6 +214,43 @@ __device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d_tmem, uint64_t adesc
         "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
         ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
         : "memory");
+}
+
+// The same with the descriptors as 32-bit halves: `alo` and `blo` hold a
+// sw128_desc's start address in 16-byte units (the other low bits are
+// constant, so a caller steps through its stages with one 32-bit add each)
+// and the high half is the same for every operand.
+constexpr uint32_t SW128_DESC_HI = (1024u >> 4) | (1u << 14) | (2u << 29);
+__device__ __forceinline__ uint32_t sw128_desc_lo(uint32_t saddr) {
+    return ((saddr >> 4) & 0x3FFFu) | (1u << 16);
+}
+__device__ __forceinline__ void tc_mma_mxf4_pair_lo(uint32_t d_tmem, uint32_t alo, uint32_t blo,
+                                                    uint32_t idesc, uint32_t accumulate,
+                                                    uint32_t sfa, uint32_t sfb) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "mov.b64 da, {%1, %7};\n\t"
+        "mov.b64 db, {%2, %7};\n\t"
+        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], da, db, %3, [%5], [%6], p;\n\t}"
+        ::"r"(d_tmem), "r"(alo), "r"(blo), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb),
+        "r"(SW128_DESC_HI)
+        : "memory");
+}
+
+// One lane of a converged warp.  The SM-pair kernels' issue loops run in all
+// 32 lanes, with only the tcgen05 instructions under this predicate, so that
+// their operands come from warp-uniform values: issuing a stage's four MMAs
+// takes 185 cycles (clock64 around them) against 320 in a loop run by lane 0
+// alone, of the 657 a 256 x 240 stage takes on a busy chip.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t x;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "elect.sync _|p, 0xffffffff;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(x));
+    return x != 0u;
 }
 
 // TMEM allocation by one warp (CG = 1: this CTA; 2: the CTA pair, issued by
