@@ -316,10 +316,16 @@ int launch_counts(qld_ctx *c, const Task &t, int b0, int b1, float *r2, long lon
                        "4-bit tensor-core kernel needs K*64 <= %d samples (K=%d)",
                        kMxf4MaxSamples, t.K);
     const KernelShape &ks = shape_of(c, variant, t, b0, b1);
+    // a launch whose tiles all run at once: smaller tiles, words split over pairs
+    SplitPlan sp{};
+    const bool split = &ks == &kMxf4PairShape && c->sm_pair == 0 &&
+                       plan_split(RowTiles{t.m, b0, b1, 0, t.symmetric, t.band}, t.K, c->r2_mode,
+                                  &sp);
     CUtensorMap tmA, tmB;
     int rc;
     if ((rc = make_tmap(c, &tmA, t.A, t.m, t.K, t.lda, ks.box_words, ks.box_rows_a, ks.swizzle)) ||
-        (rc = make_tmap(c, &tmB, t.B, t.n, t.K, t.ldb, ks.box_words, ks.box_rows_b, ks.swizzle)))
+        (rc = make_tmap(c, &tmB, t.B, t.n, t.K, t.ldb, ks.box_words,
+                        split ? sp.bn / 2 : ks.box_rows_b, ks.swizzle)))
         return rc;
     const int tb0 = b0 / ks.bn;
     const int tiles_b = (b1 - b0 + ks.bn - 1) / ks.bn;
@@ -339,6 +345,21 @@ int launch_counts(qld_ctx *c, const Task &t, int b0, int b1, float *r2, long lon
     }
     p.status = c->d_status;
     p.timeout_cycles = c->timeout_cycles;
+    if (split) {
+        p.n = b1;                        // its tile rows need not end at b1
+        cudaEvent_t e1 = nullptr;
+        if ((rc = prof_begin(c, st, &e1))) return rc;
+        const cudaError_t e =
+            launch_mxf4_split(tmA, tmB, p, RowTiles{t.m, b0, b1, sp.bn, t.symmetric, t.band},
+                              sp.ks, c->r2_mode, st);
+        if (e != cudaSuccess)
+            return set_err(c, QLD_ERR_CUDA, "counts kernel launch failed: %s", cudaGetErrorString(e));
+        if (e1) CUDA_TRY(c, cudaEventRecord(e1, st));
+        c->stats.counts_launches++;
+        c->stats.kernel_launches++;
+        c->stats.last_kernel = variant;
+        return QLD_OK;
+    }
     for (int done = 0; done < tiles_b; done += 65535) {
         const int nb = tiles_b - done < 65535 ? tiles_b - done : 65535;
         p.tb0 = tb0 + done;
@@ -1516,7 +1537,8 @@ int qld_cuda_autotune(qld_ctx *c, int m, int n, int K, int symmetric, int *kerne
         for (const Cand &cd : cands) {
             c->kernel = cd.kernel;
             c->mma_tile = cd.kernel == QLD_KERNEL_MMA ? cd.option : 0;
-            c->sm_pair = cd.kernel == QLD_KERNEL_FP4 ? cd.option : 0;
+            // option 2 is measured as the automatic choice runs it (0)
+            c->sm_pair = cd.kernel == QLD_KERNEL_FP4 && cd.option == 1 ? 1 : 0;
             // one warm-up launch, then the mean of three
             if ((rc = launch_counts(c, t, 0, nt, r2, mt, nullptr, 0, 0, c->stream)) ||
                 (rc = finish(c, c->stream)))

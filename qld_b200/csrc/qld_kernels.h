@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "qld_cuda.h"
+#include "mxf4_tiles.cuh"
 #include "qld_device.cuh"
 
 namespace qld {
@@ -46,6 +47,15 @@ cudaError_t launch_mxf4(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
 extern const KernelShape kMxf4PairShape;
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              int tiles_b, int r2_mode, cudaStream_t st);
+
+// The same arithmetic for a launch whose tiles all run at once: 256 x bn
+// tiles, each on a cluster of ks SM pairs that split its words.  plan_split
+// picks both for the tiles of `tl` (its bn is ignored); false: they do not
+// all run at once, use the persistent kernel.
+struct SplitPlan { int bn, ks; };
+bool plan_split(const RowTiles &tl, int K, int r2_mode, SplitPlan *plan);
+cudaError_t launch_mxf4_split(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
+                              const RowTiles &tl, int ks, int r2_mode, cudaStream_t st);
 
 // One task of a batched launch: its tensor maps (kBatchShape boxes), sizes,
 // output, and the number of work items (output tiles) of the tasks before it.
