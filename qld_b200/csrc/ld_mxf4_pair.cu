@@ -42,6 +42,7 @@
 // timeout, and the TMEM is released only after the last MMA has completed.
 #include "epilogue.cuh"
 #include "mxf4_rows.cuh"
+#include "mxf4_tiles.cuh"
 #include "qld_kernels.h"
 #include "tcgen05.cuh"
 
@@ -51,7 +52,7 @@ namespace {
 
 using namespace tc;
 
-constexpr int BM = 256, BN = 240;        // output tile of a pair
+constexpr int BM = RowTiles::BM, BN = 240;        // output tile of a pair
 constexpr int HM = 128, HN = 120;        // A and B rows held by each CTA
 constexpr int PW = 8;                    // packed words per row per packed stage
 constexpr int SUB = 2;                   // unpacked stages (256 samples) per packed stage
@@ -103,10 +104,12 @@ static_assert(sizeof(float2) == 8, "ColsF entry");
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
 static_assert(TASKS == 2 && SUB == 2 && UST % 2 == 0 && EPILOGUE == COLS_N, "work split");
 
-template <int MODE>
+// BAND: a band's launch (its window and tiles); otherwise two regions or a
+// single region.  One kernel for both ran the other two 1.2 % slower.
+template <int MODE, bool BAND>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-               const LdParams p, const int tiles_b) {
+               const LdParams p, const RowTiles all, const int ntiles) {
     using L = Smem<MODE>;
     constexpr int PST = L::PST;
     extern __shared__ uint8_t smem_raw[];
@@ -124,9 +127,9 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
     const uint32_t rank = cluster_rank();
     const int pair = (int)cluster_id_x(), npairs = (int)cluster_count_x();
-    const TileList<BM, BN> tl{(p.m + BM - 1) / BM, p.tb0, tiles_b, p.symmetric, p.band};
-    const int dlo = diag_lo(p.symmetric, p.band), dhi = diag_hi(p.band);
-    const int ntiles = tl.count();
+    RowTiles tl = all;
+    if (!BAND) tl.band = 0;
+    const int dlo = diag_lo(p.symmetric, tl.band), dhi = diag_hi(tl.band);
     const int my_tiles = pair < ntiles ? (ntiles - pair + npairs - 1) / npairs : 0;
 
     const int tid = threadIdx.x;
@@ -174,9 +177,9 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             int gp = 0, cur_t = 0, cur_base = 0;
             bool ok = true;
             for (int i = 0; i < my_tiles && ok; ++i) {
-                int ta, tb;
-                tl.decode_from(pair + i * npairs, ta, tb, cur_t, cur_base);
-                const int ra = ta * BM + (int)rank * HM, rb = tb * BN + (int)rank * HN;
+                int a_row, b_row;
+                tl.decode_from(pair + i * npairs, a_row, b_row, cur_t, cur_base);
+                const int ra = a_row + (int)rank * HM, rb = b_row + (int)rank * HN;
                 for (int kp = 0; kp < np; ++kp, ++gp) {
                     const int s = gp % PST;
                     if (gp >= PST && !mbar_wait(smem_u32(&pempty[s]), ((gp / PST) - 1) & 1,
@@ -290,11 +293,11 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         bool failed = false;
         int cur_t = 0, cur_base = 0;
         for (int it = 0; it < my_tiles; ++it) {
-            int ta, tb;
-            tl.decode_from(pair + it * npairs, ta, tb, cur_t, cur_base);
+            int a_row, b_row;
+            tl.decode_from(pair + it * npairs, a_row, b_row, cur_t, cur_base);
             const int ab = it & 1;
             {   // every column factor the chunks read; 0 past the tile and the task
-                const int b = tb * BN + et;
+                const int b = b_row + et;
                 const uint32_t cb = (et < BN && b < p.n) ? p.bcB[b] : 0u;
                 if constexpr (MODE == R2_EXACT)
                     epi::store_col_f32(colsf, et, cb, p.S);
@@ -312,14 +315,14 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (ready) {
                 __syncwarp();
                 tc_fence_after();
-                const int a = ta * BM + (int)rank * HM + q * 32 + lane;
+                const int a = a_row + (int)rank * HM + q * 32 + lane;
                 const bool a_ok = a < p.m;
                 const uint32_t ca = a_ok ? p.bcA[a] : 0u;
                 const epi::ARowR ra = epi::make_arow_ref(ca, p.S);
                 const epi::ARowF raf = epi::make_arow_f32(ca, p.S);
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                const int n_tile = tb * BN + BN < p.n ? tb * BN + BN : p.n;
+                const int n_tile = b_row + BN < p.n ? b_row + BN : p.n;
                 // 16-column chunks: fewer live registers than 32 (2.41 / 2.66 ms
                 // against 2.43 / 2.75 ms, exact / reference r^2), the tile's 15
 #pragma unroll 1
@@ -329,11 +332,11 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     tc_ld_32x32b_x16(tbase + (uint32_t)(c * 16), v);
                     if constexpr (MODE == R2_EXACT) {
                         epi::chunk_f32<16>(v, tbase + (uint32_t)(c * 16), raf, colsf, c * 16,
-                                           tb * BN + c * 16, a, a_ok, n_tile,
+                                           b_row + c * 16, a, a_ok, n_tile,
                                            dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
                     } else {
                         // the F32 accumulators hold the counts as floats
-                        epi::chunk_ref<0, true, 16>(v, ra, colsr, c * 16, tb * BN + c * 16, a, a_ok,
+                        epi::chunk_ref<0, true, 16>(v, ra, colsr, c * 16, b_row + c * 16, a, a_ok,
                                             n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc,
                                             p.out_row0, p.S);
                     }
@@ -366,10 +369,10 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 
 int g_max_pairs = 0;
 
-template <int MODE>
+template <int MODE, bool BAND>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                         int tiles_b, cudaStream_t st) {
-    auto kern = k_ld_mxf4_pair<MODE>;
+    auto kern = k_ld_mxf4_pair<MODE, BAND>;
     cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<MODE>::BYTES);
     if (e != cudaSuccess) return e;
@@ -390,11 +393,13 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
         }
         g_max_pairs = n;
     }
-    const long long ntiles =
-        TileList<BM, BN>{(p.m + BM - 1) / BM, p.tb0, tiles_b, p.symmetric, p.band}.count();
+    const long long last = ((long long)p.tb0 + tiles_b) * BN;
+    const RowTiles tl{p.m,         p.tb0 * BN, last < p.n ? (int)last : p.n, BN,
+                      p.symmetric, p.band};
+    const int ntiles = tl.count();
     if (ntiles == 0) return cudaSuccess;
-    const int pairs = (int)(ntiles < g_max_pairs ? ntiles : g_max_pairs);
-    kern<<<2 * pairs, THREADS, Smem<MODE>::BYTES, st>>>(tmA, tmB, p, tiles_b);
+    const int pairs = ntiles < g_max_pairs ? ntiles : g_max_pairs;
+    kern<<<2 * pairs, THREADS, Smem<MODE>::BYTES, st>>>(tmA, tmB, p, tl, ntiles);
     return cudaGetLastError();
 }
 
@@ -405,8 +410,11 @@ const KernelShape kMxf4PairShape = {BM, BN, PW, HM, HN, 64};
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              int tiles_b, int r2_mode, cudaStream_t st) {
     if (tiles_b <= 0 || p.m <= 0) return cudaSuccess;
-    return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE>(tmA, tmB, p, tiles_b, st)
-                                   : launch_mode<R2_EXACT>(tmA, tmB, p, tiles_b, st);
+    if (p.band > 0)
+        return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE, true>(tmA, tmB, p, tiles_b, st)
+                                       : launch_mode<R2_EXACT, true>(tmA, tmB, p, tiles_b, st);
+    return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE, false>(tmA, tmB, p, tiles_b, st)
+                                   : launch_mode<R2_EXACT, false>(tmA, tmB, p, tiles_b, st);
 }
 
 }  // namespace qld
