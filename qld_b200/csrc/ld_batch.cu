@@ -26,7 +26,7 @@
 //
 // Roles per CTA (576 threads in R2_EXACT, 704 in R2_REFERENCE): warp 0 queue
 // (rank 0) and TMA of the CTA's rows, warp 1 TMEM and (rank 0) the MMAs,
-// warps 2-9 unpack in two groups taking alternate 256-sample stages (each
+// warps 2-9 unpack in four groups taking the 256-sample stages in turn (each
 // thread whole rows), warps 10-17 (10-21) epilogue, two (three) per TMEM lane
 // quarter.  TMEM: two 240-column accumulators
 // (columns 0 and 256), so a tile's epilogue overlaps the next tile's MMAs,
@@ -48,17 +48,18 @@ constexpr int BM = 256, BN = 240;           // work item: output tile of a pair
 constexpr int HM = 128, HN = 120;           // A and B rows held by each CTA
 constexpr int PW = 8;                       // packed words per row per packed stage
 constexpr int SUB = 2;                      // unpacked stages (256 samples) per packed stage
-constexpr int UST = 4;                      // two unpacked stages per unpack group
+constexpr int UST = 4;                      // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;       // 8 KB
-constexpr int PB_TX = HN * PW * 8;          // 7.5 KB delivered per stage
-constexpr int PB_BYTES = 8192;              // stage stride, 1024-byte aligned
+constexpr int P_TX = (HM + HN) * PW * 8;    // 15.5 KB delivered per stage
+constexpr int P_BYTES = 16384;              // stage stride: A rows, then B rows
 constexpr int UA_BYTES = HM * 128;          // 16 KB: 256 E2M1 per row
-constexpr int UB_BYTES = HN * 128;          // 15 KB
-constexpr int UNPACK_WARPS = 8;
-constexpr int GROUP_THREADS = UNPACK_WARPS * 32 / 2;
+constexpr int U_BYTES = (HM + HN) * 128;    // 31 KB: A rows, then B rows
+constexpr int GROUPS = 4, GROUP_WARPS = 2;  // as ld_mxf4_pair.cu
+constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS;
+constexpr int GROUP_THREADS = GROUP_WARPS * 32;
 constexpr int FIRST_UNPACK_WARP = 2;
 constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
-constexpr int NROWS = HM + HN;                                // row tasks per stage
+constexpr int NROWS = HM + HN;                                // rows per stage
 constexpr int TASKS = (NROWS + GROUP_THREADS - 1) / GROUP_THREADS;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_STRIDE = 256;
@@ -90,11 +91,9 @@ struct Roles {
 template <int MODE>
 struct Smem {
     static constexpr int PST = 6;                          // packed stages in flight
-    static constexpr int OFF_UA = 0;
-    static constexpr int OFF_UB = OFF_UA + UST * UA_BYTES;
-    static constexpr int OFF_PA = OFF_UB + UST * UB_BYTES;
-    static constexpr int OFF_PB = OFF_PA + PST * PA_BYTES;
-    static constexpr int OFF_ROWS = OFF_PB + PST * PB_BYTES;
+    static constexpr int OFF_U = 0;
+    static constexpr int OFF_P = OFF_U + UST * U_BYTES;
+    static constexpr int OFF_ROWS = OFF_P + PST * P_BYTES;
     static constexpr int ROWS_BYTES = COLS_N * (MODE == R2_EXACT ? 8 : epi::COLR_BYTES);
     static constexpr int OFF_ITEMS = OFF_ROWS + ROWS_BYTES;
     static constexpr int OFF_BAR = OFF_ITEMS + QSLOTS * 16;
@@ -102,12 +101,15 @@ struct Smem {
     static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
-    static_assert(OFF_UB % 1024 == 0 && UB_BYTES % 1024 == 0 && OFF_PA % 1024 == 0 &&
-                      OFF_PB % 1024 == 0 && PB_TX <= PB_BYTES && OFF_ITEMS % 16 == 0,
+    static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
+                      P_TX <= P_BYTES && OFF_ITEMS % 16 == 0,
                   "swizzled stages must start on 1024-byte boundaries");
+    // group g takes sub-stage g % 2 of packed stages g / 2, g / 2 + 2, ...: a
+    // slot always belongs to the same two groups
+    static_assert(PST % 2 == 0 && GROUPS == 2 * SUB && GROUPS <= UST, "stage rings");
 };
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
-static_assert(TASKS == 2 && SUB == 2 && UST % 2 == 0, "work split");
+static_assert(SUB == 2, "work split");
 
 struct Item {
     int job, ta, tb, np;   // job < 0: end of the queue
@@ -169,10 +171,10 @@ k_ld_batch(const BatchParams bp) {
     if (tid == 0) {
         for (int s = 0; s < PST; ++s) {
             mbar_init(smem_u32(&pfull[s]), 1);
-            mbar_init(smem_u32(&pempty[s]), UNPACK_WARPS);   // both groups, once each
+            mbar_init(smem_u32(&pempty[s]), SUB * GROUP_WARPS);   // one group per sub-stage
         }
         for (int s = 0; s < UST; ++s) {
-            mbar_init(smem_u32(&ufull[s]), UNPACK_WARPS);    // one group in each CTA
+            mbar_init(smem_u32(&ufull[s]), 2 * GROUP_WARPS);      // one group in each CTA
             mbar_init(smem_u32(&uempty[s]), 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -245,9 +247,10 @@ k_ld_batch(const BatchParams bp) {
                         break;
                     }
                     const uint32_t fb = smem_u32(&pfull[s]);
-                    mbar_arrive_expect_tx(fb, PA_BYTES + PB_TX);
-                    tma_load_2d(smem_u32(smem + L::OFF_PA + s * PA_BYTES), &J.tmA, kp * PW, ra, fb);
-                    tma_load_2d(smem_u32(smem + L::OFF_PB + s * PB_BYTES), &J.tmB, kp * PW, rb, fb);
+                    const uint32_t dst = smem_u32(smem + L::OFF_P + s * P_BYTES);
+                    mbar_arrive_expect_tx(fb, P_TX);
+                    tma_load_2d(dst, &J.tmA, kp * PW, ra, fb);
+                    tma_load_2d(dst + PA_BYTES, &J.tmB, kp * PW, rb, fb);
                 }
                 if (rank == 1) {
                     release_item(qi);
@@ -264,8 +267,7 @@ k_ld_batch(const BatchParams bp) {
         // ------------------------------------------- MMA issuer (rank 0) --
         if (rank == 0) {
             const uint32_t sf = tmem + SF_COL;
-            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UA));
-            const uint32_t b_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UB));
+            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_U));
             uint32_t s = 0, ph = 0;      // unpacked stage and its phase
             int it_n = 0;
             bool ok = true;
@@ -296,7 +298,7 @@ k_ld_batch(const BatchParams bp) {
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t da = a_lo + s * (UA_BYTES >> 4), db = b_lo + s * (UB_BYTES >> 4);
+                    const uint32_t da = a_lo + s * (U_BYTES >> 4), db = da + (UA_BYTES >> 4);
                     if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
@@ -319,13 +321,9 @@ k_ld_batch(const BatchParams bp) {
         }
     } else if (warp < FIRST_EPI_WARP) {
         // --------------------------------------------------------- unpack --
-        // group g takes sub-stage g of every packed stage
-        const int grp = (warp - FIRST_UNPACK_WARP) / (UNPACK_WARPS / 2);
-        const int wt = ((warp - FIRST_UNPACK_WARP) % (UNPACK_WARPS / 2)) * 32 + lane;
-        mxf4rows::RowTask task[TASKS];
-#pragma unroll
-        for (int j = 0; j < TASKS; ++j)   // over 128 A + 120 B rows
-            task[j] = mxf4rows::make_task<HM>(wt + j * GROUP_THREADS, NROWS);
+        const int grp = (warp - FIRST_UNPACK_WARP) / GROUP_WARPS;
+        const mxf4rows::RowLane<GROUP_THREADS> rows(
+            ((warp - FIRST_UNPACK_WARP) % GROUP_WARPS) * 32 + lane);
         int gp = 0;
         bool ok = true;
         for (int qi = 0; ok; ++qi) {
@@ -337,6 +335,7 @@ k_ld_batch(const BatchParams bp) {
             const Item it = items[qi % QSLOTS];
             if (it.job < 0) break;
             for (int kp = 0; kp < it.np; ++kp, ++gp) {
+                if ((gp & 1) != grp / SUB) continue;
                 const int ps = gp % PST;
                 const bool got = mbar_wait(smem_u32(&pfull[ps]), (gp / PST) & 1, limit, bp.status);
                 if (!__all_sync(0xffffffffu, got)) {
@@ -344,7 +343,7 @@ k_ld_batch(const BatchParams bp) {
                     ok = false;
                     break;
                 }
-                const int gu = gp * SUB + grp;
+                const int gu = gp * SUB + grp % SUB;
                 const int us = gu % UST;
                 const bool freed = gu < UST || mbar_wait(smem_u32(&uempty[us]),
                                                          ((gu / UST) - 1) & 1, limit, bp.status);
@@ -353,11 +352,9 @@ k_ld_batch(const BatchParams bp) {
                     ok = false;
                     break;
                 }
-                const uint8_t *pa = smem + L::OFF_PA + ps * PA_BYTES;
-                const uint8_t *pb = smem + L::OFF_PB + ps * PB_BYTES;
-                uint8_t *ua = smem + L::OFF_UA + us * UA_BYTES;
-                uint8_t *ub = smem + L::OFF_UB + us * UB_BYTES;
-                mxf4rows::unpack_rows(task, pa, pb, ua, ub, grp);
+                mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(
+                    rows, NROWS, smem + L::OFF_P + ps * P_BYTES, smem + L::OFF_U + us * U_BYTES,
+                    grp % SUB);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {

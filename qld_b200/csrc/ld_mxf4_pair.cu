@@ -14,7 +14,7 @@
 // the MMAs fill the other, and each SM's shared memory supplies every
 // unpacked row once per MMA.
 //
-// Roles (both CTAs of a pair, 640 threads):
+// Roles (both CTAs of a pair, 576 threads):
 //   warp 0       TMA producer: the CTA's 128 A rows and 120 B rows, 8 packed
 //                words (512 samples) per stage, 64-byte swizzle.
 //   warp 1       TMEM allocation for the pair (cta_group::2); in rank 0 the
@@ -23,17 +23,21 @@
 //                "empty" barrier in both CTAs.  The whole warp runs the issue
 //                loop (tcgen05.cuh, elect_one): single region 2.39 -> 2.375
 //                ms, band of 5,000 over 24,000 x 100,000 3.45 -> 3.39 ms.
-//   warps 2-11   unpack (w -> four words of nibbles, as ld_mxf4.cu) into the
-//                CTA's stage; they arrive on rank 0's "full" barrier.  Two
-//                groups of five warps take alternate unpacked stages (each
-//                thread one or two rows of every other stage): two stages in
-//                flight per CTA, which the per-warp latency of a stage (load,
-//                spread, store, proxy fence, remote arrive) needs to keep up
-//                with the MMAs.  Five warps per group measured 3 % faster than
-//                four (2.44 / 2.76 ms against 2.52 / 2.83 ms, exact /
-//                reference r^2); six, at the 80 registers 22 warps leave, 4 %
-//                slower.
-//   warps 12-19  epilogue: warp w reads TMEM lane quarter w % 4 of the
+//   warps 2-9    unpack (w -> four words of nibbles, mxf4_rows.cuh) into the
+//                CTA's stage; they arrive on rank 0's "full" barrier.  Four
+//                groups of two warps take the unpacked stages in turn.  A
+//                group's steps for a stage are one serial chain (wait for the
+//                packed data and for the free buffer, load, spread, store,
+//                proxy fence, arrive: ~1,250 cycles by clock64), so two groups
+//                (of five warps) handed a stage over only every ~650 cycles,
+//                whatever the tensor cores and shared memory allowed; with
+//                four a stage takes ~600, at the shared-memory bound (620
+//                wavefronts).  Single region 2.36 -> 2.12 ms (first 100
+//                launches; 2.41 -> 2.21 in a power-capped loop), 5,000-wide
+//                band 3.26 -> 2.80 ms, 9,001 x 7,003 x 16,622 reference mode
+//                with counts 403 -> 349 us.  Three groups of three: 2.16 ms /
+//                2.85 / 367; four of three (80 registers): 2.13 / 2.82 / 359.
+//   warps 10-17  epilogue: warp w reads TMEM lane quarter w % 4 of the
 //                accumulator buffer the tile used, every other one of its
 //                fifteen 16-column chunks, applies the r^2 epilogue (gemm_cpu.c:343-404) and
 //                stores; they arrive on rank 0's "accumulator empty" barrier.
@@ -56,20 +60,21 @@ constexpr int BM = RowTiles::BM, BN = 240;        // output tile of a pair
 constexpr int HM = 128, HN = 120;        // A and B rows held by each CTA
 constexpr int PW = 8;                    // packed words per row per packed stage
 constexpr int SUB = 2;                   // unpacked stages (256 samples) per packed stage
-constexpr int UST = 4;
+constexpr int UST = 4;                   // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;    // 8 KB
-constexpr int PB_TX = HN * PW * 8;       // 7.5 KB delivered per stage
-constexpr int PB_BYTES = 8192;           // stage stride, 1024-byte aligned
+constexpr int P_TX = (HM + HN) * PW * 8; // 15.5 KB delivered per stage
+constexpr int P_BYTES = 16384;           // stage stride: A rows, then B rows
 constexpr int UA_BYTES = HM * 128;       // 16 KB: 256 E2M1 per row
-constexpr int UB_BYTES = HN * 128;       // 15 KB
-constexpr int UNPACK_WARPS = 10, EPI_WARPS = 8;
+constexpr int U_BYTES = (HM + HN) * 128; // 31 KB: A rows, then B rows
+constexpr int GROUPS = 4, GROUP_WARPS = 2;
+constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS, EPI_WARPS = 8;
 constexpr int FIRST_UNPACK_WARP = 2;
 constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
 constexpr int EPILOGUE = EPI_WARPS * 32;
-constexpr int THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;   // 640
-constexpr int GROUP_THREADS = UNPACK_WARPS * 32 / 2;         // unpackers per stage
-constexpr int NTASK = HM + HN;                               // row tasks
-constexpr int TASKS = (NTASK + GROUP_THREADS - 1) / GROUP_THREADS;
+constexpr int THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;   // 576
+constexpr int GROUP_THREADS = GROUP_WARPS * 32;              // unpackers per stage
+constexpr int NROWS = HM + HN;                               // rows per stage
+constexpr int TASKS = (NROWS + GROUP_THREADS - 1) / GROUP_THREADS;
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_STRIDE = 256;     // accumulator buffers at columns 0 and 256
 constexpr uint32_t SF_COL = 496;         // 16 columns of scale factors
@@ -85,24 +90,25 @@ constexpr uint16_t BOTH = 0x3;           // CTA mask of a commit to both ranks
 template <int MODE>
 struct Smem {
     static constexpr int PST = 6;                          // packed stages in flight
-    static constexpr int OFF_UA = 0;
-    static constexpr int OFF_UB = OFF_UA + UST * UA_BYTES;
-    static constexpr int OFF_PA = OFF_UB + UST * UB_BYTES;
-    static constexpr int OFF_PB = OFF_PA + PST * PA_BYTES;
-    static constexpr int OFF_ROWS = OFF_PB + PST * PB_BYTES;
+    static constexpr int OFF_U = 0;
+    static constexpr int OFF_P = OFF_U + UST * U_BYTES;
+    static constexpr int OFF_ROWS = OFF_P + PST * P_BYTES;
     static constexpr int ROWS_BYTES = COLS_N * (MODE == R2_EXACT ? 8 : epi::COLR_BYTES);
     static constexpr int OFF_BAR = OFF_ROWS + ROWS_BYTES;
     static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1;
     static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
-    static_assert(OFF_UB % 1024 == 0 && UB_BYTES % 1024 == 0 && OFF_PA % 1024 == 0 &&
-                      OFF_PB % 1024 == 0 && PB_TX <= PB_BYTES,
+    static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
+                      P_TX <= P_BYTES,
                   "swizzled stages must start on 1024-byte boundaries");
+    // a group sees every (GROUPS / 2)-th packed stage or so: a slot must
+    // always belong to the same groups for its phase bit to be enough
+    static_assert(PST * SUB % GROUPS == 0 && GROUPS <= UST, "stage rings");
 };
 static_assert(sizeof(float2) == 8, "ColsF entry");
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
-static_assert(TASKS == 2 && SUB == 2 && UST % 2 == 0 && EPILOGUE == COLS_N, "work split");
+static_assert(SUB == 2 && EPILOGUE == COLS_N, "work split");
 
 // BAND: a band's launch (its window and tiles); otherwise two regions or a
 // single region.  One kernel for both ran the other two 1.2 % slower.
@@ -140,10 +146,10 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     if (tid == 0) {
         for (int s = 0; s < PST; ++s) {
             mbar_init(smem_u32(&pfull[s]), 1);
-            mbar_init(smem_u32(&pempty[s]), UNPACK_WARPS);
+            mbar_init(smem_u32(&pempty[s]), SUB * GROUP_WARPS);
         }
         for (int s = 0; s < UST; ++s) {
-            mbar_init(smem_u32(&ufull[s]), UNPACK_WARPS);   // one group in each CTA
+            mbar_init(smem_u32(&ufull[s]), 2 * GROUP_WARPS);   // one group in each CTA
             mbar_init(smem_u32(&uempty[s]), 1);
         }
         for (int b = 0; b < 2; ++b) {
@@ -189,9 +195,10 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         break;
                     }
                     const uint32_t fb = smem_u32(&pfull[s]);
-                    mbar_arrive_expect_tx(fb, PA_BYTES + PB_TX);
-                    tma_load_2d(smem_u32(smem + L::OFF_PA + s * PA_BYTES), &tmA, kp * PW, ra, fb);
-                    tma_load_2d(smem_u32(smem + L::OFF_PB + s * PB_BYTES), &tmB, kp * PW, rb, fb);
+                    const uint32_t dst = smem_u32(smem + L::OFF_P + s * P_BYTES);
+                    mbar_arrive_expect_tx(fb, P_TX);
+                    tma_load_2d(dst, &tmA, kp * PW, ra, fb);
+                    tma_load_2d(dst + PA_BYTES, &tmB, kp * PW, rb, fb);
                 }
             }
             for (int g = gp > PST ? gp - PST : 0; g < gp; ++g)
@@ -205,8 +212,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // ------------------------------------------- MMA issuer (rank 0) --
         if (rank == 0) {
             const uint32_t sf = tmem + SF_COL;
-            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UA));
-            const uint32_t b_lo = sw128_desc_lo(smem_u32(smem + L::OFF_UB));
+            const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_U));
             uint32_t s = 0, ph = 0;      // unpacked stage and its phase
             bool ok = true;
             for (int it = 0; it < my_tiles && ok; ++it) {
@@ -230,7 +236,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         break;
                     }
                     tc_fence_after();
-                    const uint32_t da = a_lo + s * (UA_BYTES >> 4), db = b_lo + s * (UB_BYTES >> 4);
+                    const uint32_t da = a_lo + s * (U_BYTES >> 4), db = da + (UA_BYTES >> 4);
                     if (elect_one()) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
@@ -250,16 +256,12 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp < FIRST_EPI_WARP) {
         // --------------------------------------------------------- unpack --
-        // group g takes the unpacked stages gu = g, g + 2, ...: sub-stage g of
-        // every packed stage
-        const int grp = (warp - FIRST_UNPACK_WARP) / (UNPACK_WARPS / 2);
-        const int wt = ((warp - FIRST_UNPACK_WARP) % (UNPACK_WARPS / 2)) * 32 + lane;
-        mxf4rows::RowTask task[TASKS];
-#pragma unroll
-        for (int j = 0; j < TASKS; ++j)   // over 128 A + 120 B rows
-            task[j] = mxf4rows::make_task<HM>(wt + j * GROUP_THREADS, NTASK);
+        // group g takes the unpacked stages gu = g, g + GROUPS, ...
+        const int grp = (warp - FIRST_UNPACK_WARP) / GROUP_WARPS;
+        const mxf4rows::RowLane<GROUP_THREADS> rows(
+            ((warp - FIRST_UNPACK_WARP) % GROUP_WARPS) * 32 + lane);
         const int total_u = my_tiles * nu;
-        for (int gu = grp; gu < total_u; gu += 2) {
+        for (int gu = grp; gu < total_u; gu += GROUPS) {
             const int gp = gu / SUB;
             const int ps = gp % PST;
             const bool got = mbar_wait(smem_u32(&pfull[ps]), (gp / PST) & 1, p.timeout_cycles,
@@ -275,13 +277,13 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (lane == 0) flag_error(p.status, ST_TIMEOUT_MMA);
                 break;
             }
-            mxf4rows::unpack_rows(task, smem + L::OFF_PA + ps * PA_BYTES, smem + L::OFF_PB + ps * PB_BYTES,
-                        smem + L::OFF_UA + us * UA_BYTES, smem + L::OFF_UB + us * UB_BYTES, grp);
+            mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(rows, NROWS, smem + L::OFF_P + ps * P_BYTES,
+                                                        smem + L::OFF_U + us * U_BYTES, gu & 1);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive_rank(smem_u32(&ufull[us]), 0);
-                mbar_arrive(smem_u32(&pempty[ps]));     // both groups: UNPACK_WARPS per stage
+                mbar_arrive(smem_u32(&pempty[ps]));     // one group per sub-stage
             }
         }
     } else {

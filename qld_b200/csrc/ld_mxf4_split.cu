@@ -72,13 +72,13 @@ constexpr int MAX_SMEM = 232448;
 
 // Shared-memory layout of a launch.
 struct Layout {
-    int ub, pb, pst, push, cols, bars, bytes;   // stage strides, then offsets
+    int u, p, pst, push, cols, bars, bytes;     // stage strides, then offsets
     __host__ __device__ Layout(int bn, int ks, int pst_) {
         const int hn = bn / 2;
-        ub = hn * 128;                              // hn is a multiple of 8
-        pb = (hn * PW * 8 + 1023) / 1024 * 1024;
+        u = (HM + hn) * 128;                        // hn is a multiple of 8
+        p = ((HM + hn) * PW * 8 + 1023) / 1024 * 1024;
         pst = pst_;
-        push = UST * (UA_BYTES + ub) + pst * (PA_BYTES + pb);
+        push = UST * u + pst * p;
         const int chunks = bn / CH;
         cols = push + (ks - 1) * ((chunks + ks - 1) / ks) * SLOT_BYTES;
         bars = cols + COLS_BYTES;
@@ -104,8 +104,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     const int bn = tl.bn, hn = bn / 2;
     const Layout L(bn, ks, pst);
-    uint8_t *ua = smem, *ub = ua + UST * UA_BYTES;
-    uint8_t *pa = ub + UST * L.ub, *pb = pa + pst * PA_BYTES;
+    uint8_t *unpacked = smem, *packed = smem + UST * L.u;   // A rows, then B rows, per stage
     const float *push = reinterpret_cast<const float *>(smem + L.push);
     uint64_t *bars = reinterpret_cast<uint64_t *>(smem + L.bars);
     uint64_t *pfull = bars, *pempty = pfull + MAX_PST;
@@ -178,9 +177,10 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     break;
                 }
                 const uint32_t fb = smem_u32(&pfull[s]);
+                const uint32_t dst = smem_u32(packed + s * L.p);
                 mbar_arrive_expect_tx(fb, PA_BYTES + (uint32_t)(hn * PW * 8));
-                tma_load_2d(smem_u32(pa + s * PA_BYTES), &tmA, (kp0 + gp) * PW, rowa, fb);
-                tma_load_2d(smem_u32(pb + s * L.pb), &tmB, (kp0 + gp) * PW, rowb, fb);
+                tma_load_2d(dst, &tmA, (kp0 + gp) * PW, rowa, fb);
+                tma_load_2d(dst + PA_BYTES, &tmB, (kp0 + gp) * PW, rowb, fb);
             }
             for (int g = gp > pst ? gp - pst : 0; g < gp; ++g)
                 if (!mbar_wait(smem_u32(&pfull[g % pst]), (g / pst) & 1, kDrainCycles, nullptr)) {
@@ -195,8 +195,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const uint32_t sf = tmem + SF_COL;
             const uint32_t even = idesc_mxf4_sf(BM, bn, 0), odd = idesc_mxf4_sf(BM, bn, 2);
             const uint16_t both = (uint16_t)(0x3u << leader);
-            const uint32_t a_lo = sw128_desc_lo(smem_u32(ua)), b_lo = sw128_desc_lo(smem_u32(ub));
-            const uint32_t b_step = (uint32_t)L.ub >> 4;
+            const uint32_t a_lo = sw128_desc_lo(smem_u32(unpacked));
+            const uint32_t step = (uint32_t)L.u >> 4;
             for (int u = 0; u < nu; ++u) {
                 const uint32_t s = (uint32_t)u % UST;
                 const bool full = mbar_wait(smem_u32(&ufull[s]), (u / UST) & 1, p.timeout_cycles,
@@ -206,7 +206,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     break;
                 }
                 tc_fence_after();
-                const uint32_t da = a_lo + s * (UA_BYTES >> 4), db = b_lo + s * b_step;
+                const uint32_t da = a_lo + s * step, db = da + (UA_BYTES >> 4);
                 if (elect_one()) {
 #pragma unroll
                     for (int kk = 0; kk < 4; ++kk)
@@ -234,11 +234,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         else ra = epi::make_arow_ref(ca, p.S);
 
         const int grp = (warp - FIRST_WORKER) / GROUP_WARPS;
-        const int row = ((warp - FIRST_WORKER) % GROUP_WARPS) * 32 + lane;
-        mxf4rows::RowTask task[TASKS];
-#pragma unroll
-        for (int j = 0; j < TASKS; ++j)
-            task[j] = mxf4rows::make_task<HM>(row + j * GROUP_WARPS * 32, HM + hn);
+        const mxf4rows::RowLane<GROUP_WARPS * 32> rows(
+            ((warp - FIRST_WORKER) % GROUP_WARPS) * 32 + lane);
         bool ok = true;
         int gp = 0, ps = 0, pph = 0;               // packed stage: index, slot, phase
         for (int u = grp; u < nu; u += GROUPS) {
@@ -258,8 +255,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 ok = false;
                 break;
             }
-            mxf4rows::unpack_rows(task, pa + ps * PA_BYTES, pb + ps * L.pb, ua + us * UA_BYTES,
-                                  ub + us * L.ub, u & 1);
+            mxf4rows::unpack_rows<GROUP_WARPS * 32, TASKS>(rows, HM + hn, packed + ps * L.p,
+                                                           unpacked + us * L.u, u & 1);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
