@@ -9,18 +9,42 @@
 // reduces per word to
 //     st = popc(st | S_k),  S_k bit 0: ~a & ~b != 0   bit 1: ~a & b != 0
 //                           bit 2:  a & ~b != 0   bit 3:  a & b != 0
-// so each pair costs a few LOP3s, compares and one POPC per word -- a
-// sequential fold over the words, not a contraction, so it stays on the
-// CUDA cores.  Every word 0..K-1 counts, the zero tail bits of the last one
-// included (they are state 00, as in the reference); words past K do not.
+// Every word 0..K-1 counts, the zero tail bits of the last one included (they
+// are state 00, as in the reference); words past K do not.
 //
-// Structure as ld_popc.cu: one CTA per 128 x 128 output tile, a TMA producer
-// warp staging 128 rows x 16 words (128-byte swizzle) of A and of B per stage,
-// and 8 consumer warps of 16 x 16 threads, each folding an 8 x 8 block of
-// pairs (A rows tx + 16i, B rows ty + 16j).  Output: one byte per pair,
-// st[(b - out_row0) * lds + a], inside the diagonal window (single region:
-// a >= b).  Every wait is bounded; on expiry the kernel records the cause in
-// the status word and returns.
+// A word maps the four values st can have after any word (1..4) to fewer:
+// S = {00,01,10} makes it 3 and all four states make it 4 whatever came
+// before, and most pairs of other words leave one value as well (f_S of 1..4
+// for S = 1, 3, 5, 7, 15: 1,2,2,2 / 2,2,2,3 / 2,3,3,2 / 3,3,3,3 / 4,4,4,4).
+// So the fold is evaluated from the END of the rows: F, four bytes, holds the
+// final state for each value st may have before the words seen so far, and
+// the word before them makes it F o f_S -- one byte permutation of F, whose
+// selector is a sum of four terms (below).  A pair whose four bytes have
+// become one value is finished, however long its rows are.  A tile takes
+//   1. the last 4 words of all its pairs;
+//   2. the remaining pairs (of founder haplotypes with 1 % noise, 1.3 %), up to
+//      1,024, one by one towards the start, up to 64 words each, spread over
+//      the threads;
+//   3. for what remains (rows that are zero almost everywhere), one pass over
+//      the remaining words of its 256 rows: if neither row has a bit there,
+//      the state before the words seen is 1; if one has but every word still
+//      contains state 00 (the largest word popcounts add up to less than 64),
+//      it is 2, 3 or 4, which often suffices;
+//   4. the next 16 words of all pairs, then 64, and so on to the start.
+// Word 0 is entered with st = 0, so its map gives every byte F(popc(S)) and
+// settles every pair.  The results are the same for any input, and rows that
+// defeat every shortcut cost one walk over all their words.
+//
+// Bound by integer issue: ~19 instructions per pair and word, 9.8 us per word
+// of a 4,001-SNP single region, over 4 words instead of K.  4,001 SNPs x
+// 16,622 samples (K = 260) of founder haplotypes with 1 % noise: 2,367 us with
+// one POPC per pair and word over all words, 64 now; one bit per row: 211;
+// dense random rows: 52; rows built to defeat every shortcut (all ones): 2,540.
+//
+// One CTA per 128 x 128 tile, 256 threads: lane l holds A rows l + 32 i, warp
+// w B rows 16 w + j, a thread 4 x 16 pairs, so a store writes 32 consecutive
+// bytes.  Output: one byte per pair, st[(b - out_row0) * lds + a], inside the
+// diagonal window (single region: a >= b).
 #include "qld_device.cuh"
 #include "qld_kernels.h"
 
@@ -29,152 +53,203 @@ namespace qld {
 namespace {
 
 constexpr int BM = 128, BN = 128;
-constexpr int KC = 16;
-constexpr int TILE_BYTES = BM * KC * 8;
-constexpr int CONSUMERS = 256;
-constexpr int THREADS = CONSUMERS + 32;
-constexpr int STAGES = 4;
+constexpr int THREADS = 256;
+constexpr int NI = 4, NJ = 16;           // A and B rows of a thread
+constexpr int W = 4;                     // words per chunk, and of the first walk
+constexpr int LIST = 1024;               // remaining pairs walked one by one
+constexpr int LIST_WORDS = 64;           // words each of them may take
+constexpr uint32_t START = 0x04030201u;  // F before any word
 
-// Joint states present in one 64-bit word pair, given as 32-bit halves.
-__device__ __forceinline__ uint32_t word_states(uint32_t alo, uint32_t ahi, uint32_t blo,
-                                                uint32_t bhi) {
-    const uint32_t s11 = (alo & blo) | (ahi & bhi);
-    const uint32_t s10 = (alo & ~blo) | (ahi & ~bhi);
-    const uint32_t s01 = (~alo & blo) | (~ahi & bhi);
-    const uint32_t s00 = ~(alo | blo) | ~(ahi | bhi);
-    return (s00 != 0u ? 1u : 0u) | (s01 != 0u ? 2u : 0u) | (s10 != 0u ? 4u : 0u) |
-           (s11 != 0u ? 8u : 0u);
+// F o f_S for one word pair (32-bit halves).  Byte i of the result is byte
+// f_S(i + 1) - 1 of F, and f_S(v) = popc(v | S) = popc(S) + popc(v & ~S): as a
+// permutation selector, state 00 adds 1 to every nibble if present and to
+// those of v = 1 and 3 if not, 01 likewise v = 2 and 3, 10 v = 4, 11 none.
+// `entry` is all ones, or zero for word 0, whose v = 0 has no bit to add.
+__device__ __forceinline__ uint32_t before(uint32_t F, uint2 a, uint2 b, uint32_t entry) {
+    const uint32_t s11 = (a.x & b.x) | (a.y & b.y);
+    const uint32_t s10 = (a.x & ~b.x) | (a.y & ~b.y);
+    const uint32_t s01 = (~a.x & b.x) | (~a.y & b.y);
+    const uint32_t s00 = ~((a.x | b.x) & (a.y | b.y));
+    const uint32_t sel = (s00 != 0u ? 0x1111u : 0x0101u & entry) +
+                         (s01 != 0u ? 0x1111u : 0x0110u & entry) +
+                         (s10 != 0u ? 0x1111u : 0x1000u & entry) +
+                         (s11 != 0u ? 0u : 0u - 0x1111u);
+    return __byte_perm(F, F, sel);
 }
 
-__global__ void __launch_bounds__(THREADS, 1)
-k_states(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-         const StatesParams p) {
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t *smem = reinterpret_cast<uint8_t *>(
-        (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint8_t *sA = smem;
-    uint8_t *sB = smem + STAGES * TILE_BYTES;
-    uint64_t *full = reinterpret_cast<uint64_t *>(sB + STAGES * TILE_BYTES);
-    uint64_t *empty = full + STAGES;
+// The state if it does not depend on the words before (1..4), else 0.
+__device__ __forceinline__ uint32_t settled(uint32_t F) {
+    const uint32_t v = F & 255u;
+    return F == v * 0x01010101u ? v : 0u;
+}
 
-    const int ta = blockIdx.x;
-    const int tb = p.tb0 + blockIdx.y;
-    const int dlo = p.symmetric ? 0 : -2147483647 - 1;
-    if (p.symmetric && (long long)ta * BM + BM - 1 < (long long)tb * BN) return;
-    if (grid_failed(p.status)) return;
+__device__ __forceinline__ uint2 load_word(const uint64_t *p) {
+    return *reinterpret_cast<const uint2 *>(p);
+}
 
-    const int tid = threadIdx.x;
-    const int warp = tid >> 5, lane = tid & 31;
-    const int nk = (p.K + KC - 1) / KC;
-
-    if (tid == 0) {
-        for (int s = 0; s < STAGES; ++s) {
-            mbar_init(smem_u32(&full[s]), 1);
-            mbar_init(smem_u32(&empty[s]), CONSUMERS / 32);
-        }
-        fence_barrier_init();
-    }
-    __syncthreads();
-
-    if (warp == CONSUMERS / 32) {
-        if (lane == 0) {
-            prefetch_tmap(&tmA);
-            prefetch_tmap(&tmB);
-            int issued = 0;
-            for (int kc = 0; kc < nk; ++kc) {
-                const int s = kc % STAGES;
-                if (kc >= STAGES && !mbar_wait(smem_u32(&empty[s]), ((kc / STAGES) - 1) & 1,
-                                               p.timeout_cycles, p.status)) {
-                    flag_error(p.status, ST_TIMEOUT_EMPTY);
-                    break;
-                }
-                const uint32_t fb = smem_u32(&full[s]);
-                mbar_arrive_expect_tx(fb, 2 * TILE_BYTES);
-                tma_load_2d(smem_u32(sA + s * TILE_BYTES), &tmA, kc * KC, ta * BM, fb);
-                tma_load_2d(smem_u32(sB + s * TILE_BYTES), &tmB, kc * KC, tb * BN, fb);
-                ++issued;
-            }
-            for (int kc = issued > STAGES ? issued - STAGES : 0; kc < issued; ++kc) {
-                if (!mbar_wait(smem_u32(&full[kc % STAGES]), (kc / STAGES) & 1,
-                               kDrainCycles, nullptr)) {
-                    flag_error(p.status, ST_TIMEOUT_DRAIN);
-                    break;
-                }
-            }
-        }
-        return;
-    }
-
-    const int tx = tid & 15, ty = tid >> 4;
-    const int xa = tx & 7, xb = ty & 7;
-    uint32_t st[8][8];
+// One pair's words s0 - 1, s0 - 2, ... put before those of F, until its state is
+// settled; 0 if it is not after LIST_WORDS words.  Eight words' loads are in
+// flight at once.
+__device__ __noinline__ uint32_t walk_back(const uint64_t *a, const uint64_t *b, int s0,
+                                           uint32_t F) {
+    const int stop = s0 > LIST_WORDS ? s0 - LIST_WORDS : 0;
+    for (int k0 = s0; k0 > stop; k0 -= 8) {
+        uint2 wa[8], wb[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+        for (int q = 0; q < 8; ++q)
+            if (k0 - 1 - q >= stop) {
+                wa[q] = load_word(a + k0 - 1 - q);
+                wb[q] = load_word(b + k0 - 1 - q);
+            }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) st[i][j] = 0u;
+        for (int q = 0; q < 8; ++q)
+            if (k0 - 1 - q >= stop) F = before(F, wa[q], wb[q], k0 - 1 - q == 0 ? 0u : ~0u);
+        const uint32_t v = settled(F);
+        if (v) return v;
+    }
+    return 0u;
+}
 
-    for (int kc = 0; kc < nk; ++kc) {
-        const int s = kc % STAGES;
-        if (!mbar_wait(smem_u32(&full[s]), (kc / STAGES) & 1, p.timeout_cycles, p.status)) {
-            flag_error(p.status, ST_TIMEOUT_FULL);
-            return;
+__global__ void __launch_bounds__(THREADS, 2) k_states(const StatesParams p) {
+    __shared__ uint2 sA[W][BM], sB[W][BN];
+    __shared__ uint32_t row_info[BM + BN];   // largest word popcount of the remaining words
+    __shared__ uint32_t list_pair[LIST], list_x[LIST];
+    __shared__ uint32_t not_done[THREADS][2];
+    __shared__ int listed;
+
+    const int a0 = blockIdx.x * BM, b0 = (p.tb0 + (int)blockIdx.y) * BN;
+    if (p.symmetric && a0 + BM - 1 < b0) return;
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int my_a = a0 + lane, my_b = b0 + warp * NJ;
+    // the row this thread loads: A rows first
+    const bool is_a = tid < BM;
+    const int row = is_a ? a0 + tid : b0 + tid - BM;
+    const bool row_ok = row < (is_a ? p.m : p.n);
+    const uint64_t *row_words =
+        is_a ? p.A + (long long)row * p.lda : p.B + (long long)row * p.ldb;
+    uint2 *row_smem = is_a ? &sA[0][tid] : &sB[0][tid - BM];
+
+    // pairs the task does not have count as finished
+    uint64_t done = 0;
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) {
+            const int a = my_a + 32 * i, b = my_b + j;
+            const bool need = a < p.m && b < p.n && (!p.symmetric || a >= b);
+            done |= (uint64_t)(!need) << (j * NI + i);
         }
-        const int words = p.K - kc * KC < KC ? p.K - kc * KC : KC;   // words past K: skip
-        const uint8_t *a_base = sA + s * TILE_BYTES + tx * 128;
-        const uint8_t *b_base = sB + s * TILE_BYTES + ty * 128;
+    auto put = [&](int j, int i, uint32_t st) {
+        p.out[(long long)(my_b + j - p.out_row0) * p.lds + my_a + 32 * i] = (uint8_t)st;
+        done |= 1ull << (j * NI + i);
+    };
+
+    uint32_t x[NJ][NI];                      // F of every pair
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int i = 0; i < NI; ++i) x[j][i] = START;
+
+    long long len = W;
+    for (int end = p.K;; len *= 4) {
+        const int s0 = end > len ? (int)(end - len) : 0;
+        const bool busy = __any_sync(0xffffffffu, ~done != 0ull);
+        for (int e = end; e > s0; e -= W) {  // words [e - W, e), last first
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < W; ++w)
+                row_smem[w * BM] = row_ok && e - 1 - w >= s0 ? load_word(row_words + e - 1 - w)
+                                                             : make_uint2(0u, 0u);
+            __syncthreads();
+            if (!busy) continue;
+            const int words = e - s0 < W ? e - s0 : W;
 #pragma unroll 1
-        for (int c = 0; 2 * c < words; ++c) {
-            uint4 av[8], bv[8];
-            const int oa = (c ^ xa) << 4, ob = (c ^ xb) << 4;
+            for (int w = 0; w < words; ++w) {
+                const uint32_t entry = e - 1 - w == 0 ? 0u : ~0u;
+                uint2 a[NI];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-                av[i] = *reinterpret_cast<const uint4 *>(a_base + i * 16 * 128 + oa);
+                for (int i = 0; i < NI; ++i) a[i] = sA[w][lane + 32 * i];
 #pragma unroll
-            for (int j = 0; j < 8; ++j)
-                bv[j] = *reinterpret_cast<const uint4 *>(b_base + j * 16 * 128 + ob);
-            const bool second = 2 * c + 1 < words;
+                for (int j = 0; j < NJ; ++j) {
+                    const uint2 b = sB[w][warp * NJ + j];
 #pragma unroll
-            for (int i = 0; i < 8; ++i)
-#pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    uint32_t v = __popc(st[i][j] | word_states(av[i].x, av[i].y, bv[j].x, bv[j].y));
-                    if (second)
-                        v = __popc(v | word_states(av[i].z, av[i].w, bv[j].z, bv[j].w));
-                    st[i][j] = v;
+                    for (int i = 0; i < NI; ++i) x[j][i] = before(x[j][i], a[i], b, entry);
                 }
+            }
         }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(smem_u32(&empty[s]));
-    }
-
-    const int a0 = ta * BM + tx, b0 = tb * BN + ty;
+        end = s0;
+        // 1. the settled pairs; the others are listed
+        if (tid == 0) listed = 0;
+        not_done[tid][0] = not_done[tid][1] = 0u;
+        __syncthreads();
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-        const int b = b0 + 16 * j;
-        if (b >= p.n) break;
-        uint8_t *out = p.out + (long long)(b - p.out_row0) * p.lds;
+        for (int j = 0; j < NJ; ++j)
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int a = a0 + 16 * i;
-            if (a < p.m && a - b >= dlo) out[a] = (uint8_t)st[i][j];
+            for (int i = 0; i < NI; ++i) {
+                const int k = j * NI + i;
+                if ((done >> k) & 1ull) continue;
+                const uint32_t v = settled(x[j][i]);
+                if (v) {
+                    put(j, i, v);
+                    continue;
+                }
+                const int at = atomicAdd(&listed, 1);
+                if (at < LIST) {                 // its walker finishes it, or says so
+                    list_pair[at] = (uint32_t)(tid << 8 | k);
+                    list_x[at] = x[j][i];
+                    done |= 1ull << k;
+                }
+            }
+        __syncthreads();
+        const int entries = listed < LIST ? listed : LIST;
+        if (listed == 0) break;
+        // 2. one by one, spread over the threads
+        for (int e = tid; e < entries; e += THREADS) {
+            const int k = (int)(list_pair[e] & 255u), owner = (int)(list_pair[e] >> 8);
+            const int a = a0 + (owner & 31) + 32 * (k % NI), b = b0 + (owner >> 5) * NJ + k / NI;
+            const uint32_t v = walk_back(p.A + (long long)a * p.lda, p.B + (long long)b * p.ldb,
+                                         s0, list_x[e]);
+            if (v) p.out[(long long)(b - p.out_row0) * p.lds + a] = (uint8_t)v;
+            else atomicOr(&not_done[owner][k >> 5], 1u << (k & 31));
         }
+        __syncthreads();
+        done &= ~((uint64_t)not_done[tid][1] << 32 | not_done[tid][0]);
+        if (!__syncthreads_or(~done != 0ull)) break;
+        // 3. what the words before s0 hold, row by row
+        uint32_t most = 0;
+        if (row_ok) {
+#pragma unroll 8
+            for (int k = 0; k < s0; ++k) {
+                const uint2 v = load_word(row_words + k);
+                const uint32_t c = (uint32_t)(__popc(v.x) + __popc(v.y));
+                most = c > most ? c : most;
+            }
+        }
+        row_info[tid] = most;
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < NJ; ++j)
+#pragma unroll
+            for (int i = 0; i < NI; ++i) {
+                if ((done >> (j * NI + i)) & 1ull) continue;
+                const uint32_t ca = row_info[lane + 32 * i], cb = row_info[BM + warp * NJ + j];
+                const uint32_t F = x[j][i], v = (F >> 8) & 255u;
+                if (ca + cb == 0u) put(j, i, F & 255u);
+                else if (ca + cb < 64u && F >> 8 == v * 0x010101u) put(j, i, v);
+            }
+        if (!__syncthreads_or(~done != 0ull)) break;
     }
 }
 
 }  // namespace
 
-const KernelShape kStatesShape = {BM, BN, KC, BM, BN, 128};
-
-cudaError_t launch_states(const CUtensorMap &tmA, const CUtensorMap &tmB, const StatesParams &p,
-                          int tiles_b, cudaStream_t st) {
+cudaError_t launch_states(const StatesParams &p, int tiles_b, cudaStream_t st) {
     if (tiles_b <= 0 || p.m <= 0) return cudaSuccess;
-    const size_t smem = 1024 + 2 * STAGES * TILE_BYTES + 2 * STAGES * sizeof(uint64_t);
-    cudaError_t e =
-        cudaFuncSetAttribute(k_states, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
     dim3 grid((p.m + BM - 1) / BM, tiles_b);
-    k_states<<<grid, THREADS, smem, st>>>(tmA, tmB, p);
+    k_states<<<grid, THREADS, 0, st>>>(p);
     return cudaGetLastError();
 }
+
+const int kStatesRows = BN;
 
 }  // namespace qld

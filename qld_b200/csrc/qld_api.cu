@@ -408,25 +408,19 @@ bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 // at out[(b - out_row0) * lds + a].
 int launch_states_range(qld_ctx *c, const Task &t, int b0, int b1, uint8_t *out, long long lds,
                         int out_row0, cudaStream_t st) {
-    const KernelShape &ks = kStatesShape;
-    CUtensorMap tmA, tmB;
     int rc;
-    if ((rc = make_tmap(c, &tmA, t.A, t.m, t.K, t.lda, ks.box_words, ks.box_rows_a, ks.swizzle)) ||
-        (rc = make_tmap(c, &tmB, t.B, t.n, t.K, t.ldb, ks.box_words, ks.box_rows_b, ks.swizzle)))
-        return rc;
-    const int tb0 = b0 / ks.bn;
-    const int tiles_b = (b1 - b0 + ks.bn - 1) / ks.bn;
+    const int tb0 = b0 / kStatesRows;
+    const int tiles_b = (b1 - b0 + kStatesRows - 1) / kStatesRows;
     StatesParams p{};
-    p.m = t.m; p.n = t.n; p.K = t.K; p.symmetric = t.symmetric;
+    p.A = t.A; p.B = t.B; p.lda = t.lda; p.ldb = t.ldb;
+    p.m = t.m; p.n = b1; p.K = t.K; p.symmetric = t.symmetric;
     p.out = out; p.lds = lds; p.out_row0 = out_row0;
-    p.status = c->d_status;
-    p.timeout_cycles = c->timeout_cycles;
     for (int done = 0; done < tiles_b; done += 65535) {
         const int nb = tiles_b - done < 65535 ? tiles_b - done : 65535;
         p.tb0 = tb0 + done;
         cudaEvent_t e1 = nullptr;
         if ((rc = prof_begin(c, st, &e1))) return rc;
-        cudaError_t e = launch_states(tmA, tmB, p, nb, st);
+        cudaError_t e = launch_states(p, nb, st);
         if (e != cudaSuccess)
             return set_err(c, QLD_ERR_CUDA, "states kernel launch failed: %s",
                            cudaGetErrorString(e));

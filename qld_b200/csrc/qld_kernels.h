@@ -89,17 +89,16 @@ cudaError_t launch_batch(const BatchParams &bp, int r2_mode, int max_ctas, cudaS
 // COUNTSTATES (ld_states.cu): state value of every pair, one byte each at
 // out[(b - out_row0) * lds + a]; single region: only a >= b.
 struct StatesParams {
+    const uint64_t *A, *B;
+    long long lda, ldb;       // words between rows
     int m, n, K, symmetric;
     int tb0;                  // first B tile of this launch
     uint8_t *out;
     long long lds;
     int out_row0;
-    unsigned *status;
-    long long timeout_cycles;
 };
-extern const KernelShape kStatesShape;
-cudaError_t launch_states(const CUtensorMap &tmA, const CUtensorMap &tmB, const StatesParams &p,
-                          int tiles_b, cudaStream_t st);
+extern const int kStatesRows;   // B rows per tile
+cudaError_t launch_states(const StatesParams &p, int tiles_b, cudaStream_t st);
 
 // VCF sites -> packed rows (vcf_pack.cu).  With rnd_off NULL the launch only
 // counts: per site the random draws its unphased genotypes need
