@@ -45,6 +45,7 @@
 // cluster barriers at start and end on every path, including after a
 // timeout, and the TMEM is released only after the last MMA has completed.
 #include "epilogue.cuh"
+#include "launch_util.h"
 #include "mxf4_rows.cuh"
 #include "mxf4_tiles.cuh"
 #include "qld_kernels.h"
@@ -174,6 +175,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     // barrier initialisation and both CTAs' scale factors, cluster-wide
     cluster_sync_all();
     tc_fence_after();
+    griddep_launch();
+    griddep_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------- producer --
@@ -375,8 +378,8 @@ template <int MODE, bool BAND>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                         int tiles_b, cudaStream_t st) {
     auto kern = k_ld_mxf4_pair<MODE, BAND>;
-    cudaError_t e =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<MODE>::BYTES);
+    static std::atomic<unsigned long long> allowed;
+    cudaError_t e = allow_smem(kern, Smem<MODE>::BYTES, allowed);
     if (e != cudaSuccess) return e;
     if (g_max_pairs == 0) {
         int dev = 0, sms = 0;
@@ -401,8 +404,15 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     const int ntiles = tl.count();
     if (ntiles == 0) return cudaSuccess;
     const int pairs = ntiles < g_max_pairs ? ntiles : g_max_pairs;
-    kern<<<2 * pairs, THREADS, Smem<MODE>::BYTES, st>>>(tmA, tmB, p, tl, ntiles);
-    return cudaGetLastError();
+    cudaLaunchAttribute at = overlap_attr();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Smem<MODE>::BYTES;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, tl, ntiles);
 }
 
 }  // namespace

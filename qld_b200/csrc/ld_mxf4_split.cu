@@ -37,6 +37,7 @@
 #include <atomic>
 
 #include "epilogue.cuh"
+#include "launch_util.h"
 #include "mxf4_rows.cuh"
 #include "mxf4_tiles.cuh"
 #include "qld_kernels.h"
@@ -144,6 +145,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     tc_fence_before();
     cluster_sync_all();
     tc_fence_after();
+    griddep_launch();
+    griddep_wait();
 
     // the cluster's tile, and the pair's part of the packed words
     int a_row, b_row, t0 = 0, base = 0;
@@ -346,9 +349,19 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 // every other packed stage, so a slot must always belong to the same groups
 // for its phase bit to be enough), or 0.
 int packed_stages(int bn, int ks) {
-    int pst = MAX_PST;
-    while (pst > 0 && Layout(bn, ks, pst).bytes > MAX_SMEM) pst -= 2;
-    return pst;
+    struct Table {
+        signed char pst[MAX_BN / CH][3];
+        Table() {
+            for (int b = CH; b <= MAX_BN; b += CH)
+                for (int k = 1; k <= 4; k *= 2) {
+                    int n = MAX_PST;
+                    while (n > 0 && Layout(b, k, n).bytes > MAX_SMEM) n -= 2;
+                    pst[b / CH - 1][k >> 1] = (signed char)n;
+                }
+        }
+    };
+    static const Table table;
+    return table.pst[bn / CH - 1][ks >> 1];
 }
 
 // Clusters of 2 ks CTAs that run at once, asked of the driver once per ks.
@@ -390,19 +403,21 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     const int tiles = tl.count(), pst = packed_stages(tl.bn, ks);
     if (tiles == 0) return cudaSuccess;
     if (pst < 2) return cudaErrorInvalidConfiguration;
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM);
+    static std::atomic<unsigned long long> allowed;
+    cudaError_t e = allow_smem(kern, MAX_SMEM, allowed);
     if (e != cudaSuccess) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(tiles * 2 * ks), 1, 1);
     cfg.blockDim = dim3(THREADS, 1, 1);
     cfg.dynamicSmemBytes = (size_t)Layout(tl.bn, ks, pst).bytes;
     cfg.stream = st;
-    cudaLaunchAttribute at[1];
+    cudaLaunchAttribute at[2];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = (unsigned)(2 * ks);
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    at[1] = overlap_attr();
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, tl, ks, pst);
 }
 

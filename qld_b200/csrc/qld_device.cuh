@@ -117,6 +117,18 @@ __device__ __forceinline__ bool grid_failed(const unsigned *status) {
     return status && *((volatile const unsigned *)status) != 0u;
 }
 
+// Programmatic dependent launch.  griddep_launch: the next kernel of the stream
+// may take SMs as they become free (its blocks wait in griddep_wait).
+// griddep_wait: returns when every kernel before this one in the stream has
+// completed and its writes are visible; before it a kernel touches no global
+// memory.  A plain launch returns from it at once.
+__device__ __forceinline__ void griddep_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void griddep_wait() {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ void prefetch_tmap(const CUtensorMap *tm) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tm)) : "memory");
 }
