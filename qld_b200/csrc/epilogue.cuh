@@ -22,6 +22,53 @@
 namespace qld {
 namespace epi {
 
+// ------------------------------------------------- two columns at a time --
+//
+// Packed pairs of floats (Blackwell's f32x2 instructions): each half is
+// rounded as the scalar instruction rounds it, one issue slot for both.
+// The epilogue shares its SM's issue slots and shared-memory port with the
+// unpack, and for tables of up to ~10,000 samples it, not the MMAs, sets a
+// tile's time; in pairs of columns it takes half the arithmetic instructions
+// and half the column-factor loads.  Exact mode, with the next tile's factors
+// prefetched (ld_mxf4_pair.cu): band of 1,000 over 50,000 x 10,001 234 -> 199
+// us, single region 2.12 -> 2.07 ms, 300-task batch 576 -> 566 us.
+typedef unsigned long long f2;
+
+__device__ __forceinline__ f2 pack2(float a, float b) {
+    f2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ f2 splat2(float a) { return pack2(a, a); }
+__device__ __forceinline__ void unpack2(f2 x, float &a, float &b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x));
+}
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+    f2 r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+    f2 r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 sub2(f2 a, f2 b) {
+    f2 r;
+    asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+    f2 r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+    float r;
+    asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+    return r;
+}
+
 // ------------------------------------------- R2_REFERENCE column factors --
 //
 // One float4 per column (and per A row, in registers): x = v = fl32(c/S) as
@@ -353,37 +400,48 @@ __device__ __forceinline__ void chunk(uint32_t (&v)[32], const ARow &ra, const C
 // empty SNPs and NaN for 0/0 match the FP64 evaluation; values above 1.00009
 // (possible only when the bit counts do not match the data) are re-evaluated
 // in FP64 so the 123.456 rule decides exactly as in the other kernels.
-struct ColsF {
-    float2 *f;   // (cB as float, 1/(cB(S-cB)) rounded to float) per column
-    __device__ __forceinline__ ColsF(uint8_t *base, int) : f(reinterpret_cast<float2 *>(base)) {}
+//
+// Factors of a row or column: c and 1/(c(S-c)), the latter 0 for an empty SNP
+// (c = 0), so that its pairs come out 0 without a test.  That fails only
+// against a factor that is not a finite, non-negative number -- a fixed SNP
+// (c = S: infinity) or a bit count above S -- which `special` reports: a warp
+// that holds or meets one applies the zero rule explicitly.
+struct FactorF {
+    float c, inv;
+    bool special;
 };
 
 __device__ __forceinline__ double inv_var64(double c, double S) { return 1.0 / (c * (S - c)); }
 
-__device__ __forceinline__ void store_col_f32(const ColsF &f, int bl, uint32_t c, int S) {
-    f.f[bl] = make_float2((float)c, __double2float_rn(inv_var64((double)c, (double)S)));
-}
-
-struct ARowF {
-    float ca, inv;
-    bool zero;
-};
-
-__device__ __forceinline__ ARowF make_arow_f32(uint32_t c, int S) {
-    ARowF r;
-    r.ca = (float)c;
-    r.inv = __double2float_rn(inv_var64((double)c, (double)S));
-    r.zero = c == 0u;
+__device__ __forceinline__ FactorF factor_f32(uint32_t c, int S) {
+    FactorF r;
+    r.c = (float)c;
+    r.inv = c == 0u ? 0.0f : __double2float_rn(inv_var64((double)c, (double)S));
+    r.special = !(r.inv >= 0.0f && r.inv < __uint_as_float(0x7F800000u));
     return r;
 }
 
-__device__ __forceinline__ float pair_r2_f32(float c, float S_f, const ARowF &ra, float2 col) {
-    const float hi = __fmul_rn(ra.ca, col.x);
-    const float lo = __fmaf_rn(ra.ca, col.x, -hi);
-    const float D = __fsub_rn(__fmaf_rn(S_f, c, -hi), lo);
-    const float r = __fmul_rn(__fmul_rn(D, D), __fmul_rn(ra.inv, col.y));
-    return (ra.zero || col.x == 0.0f) ? 0.0f : r;
+// Column factors, a float4 per column pair: c, c, 1/(c(S-c)), 1/(c(S-c)).
+struct ColsF {
+    float *f;
+    __device__ __forceinline__ ColsF(uint8_t *base, int) : f(reinterpret_cast<float *>(base)) {}
+    __device__ __forceinline__ float c(int bl) const { return f[(bl >> 1) * 4 + (bl & 1)]; }
+    __device__ __forceinline__ ulonglong2 pair(int bl) const {   // bl even: {c, c}, {inv, inv}
+        return *reinterpret_cast<const ulonglong2 *>(f + bl * 2);
+    }
+};
+
+// Returns the column's `special`.
+__device__ __forceinline__ bool store_col_f32(const ColsF &f, int bl, uint32_t c, int S) {
+    const FactorF x = factor_f32(c, S);
+    f.f[(bl >> 1) * 4 + (bl & 1)] = x.c;
+    f.f[(bl >> 1) * 4 + 2 + (bl & 1)] = x.inv;
+    return x.special;
 }
+
+typedef FactorF ARowF;
+
+__device__ __forceinline__ ARowF make_arow_f32(uint32_t c, int S) { return factor_f32(c, S); }
 
 // The FP64 evaluation (pair_r2_exact) from the same exact inputs.
 __device__ __forceinline__ float pair_r2_f64(float c, float ca, float cb, int S) {
@@ -400,12 +458,13 @@ __device__ __forceinline__ float pair_r2_f64(float c, float ca, float cb, int S)
 // address the chunk was loaded from: the rare pairs whose FP32 value lies
 // above 1.00009 are re-evaluated in FP64 from their count, reloaded one
 // column at a time (warp-uniform loads, off the common path).
+// cols_special: a column of the tile is `special`.
 template <int CW = 32>
 __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, const ARowF &ra,
-                                          const ColsF &f, int bl0, int b0, int a, bool a_ok,
-                                          int n, int dlo, int dhi, float *r2, long long ldr,
-                                          uint32_t *counts, long long ldc, int row0, int S) {
-    const float S_f = (float)S;
+                                          const ColsF &f, bool cols_special, int bl0, int b0,
+                                          int a, bool a_ok, int n, int dlo, int dhi, float *r2,
+                                          long long ldr, uint32_t *counts, long long ldc, int row0,
+                                          int S) {
     if (counts && a_ok) {
 #pragma unroll
         for (int t = 0; t < CW; ++t) {
@@ -414,12 +473,25 @@ __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, con
                 counts[(long long)(b - row0) * ldc + a] = (uint32_t)__uint_as_float(v[t]);
         }
     }
+    const f2 S2 = splat2((float)S), ca = splat2(ra.c), nca = splat2(-ra.c), ia = splat2(ra.inv);
     float rmax = 0.0f;
 #pragma unroll
-    for (int t = 0; t < CW; ++t) {
-        const float r = pair_r2_f32(__uint_as_float(v[t]), S_f, ra, f.f[bl0 + t]);
-        rmax = fmaxf(rmax, r);
-        v[t] = __float_as_uint(r);
+    for (int t = 0; t < CW; t += 2) {
+        const ulonglong2 col = f.pair(bl0 + t);
+        const f2 cnt = pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1]));
+        const f2 nhi = mul2(nca, col.x);                       // -hi
+        const f2 lo = fma2(ca, col.x, nhi);
+        const f2 D = sub2(fma2(S2, cnt, nhi), lo);
+        float r0, r1;
+        unpack2(mul2(mul2(D, D), mul2(ia, col.y)), r0, r1);
+        rmax = max3(rmax, r0, r1);
+        v[t] = __float_as_uint(r0);
+        v[t + 1] = __float_as_uint(r1);
+    }
+    if (__any_sync(0xffffffffu, ra.special) || cols_special) {
+#pragma unroll
+        for (int t = 0; t < CW; ++t)
+            if (ra.c == 0.0f || f.c(bl0 + t) == 0.0f) v[t] = 0u;
     }
     if (__any_sync(0xffffffffu, rmax > 1.00009f)) {
 #pragma unroll
@@ -433,7 +505,7 @@ __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, con
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 if (redo)
                     v[t] = __float_as_uint(
-                        pair_r2_f64(__uint_as_float(w), ra.ca, f.f[bl0 + t].x, S));
+                        pair_r2_f64(__uint_as_float(w), ra.c, f.c(bl0 + t), S));
             }
         }
     }

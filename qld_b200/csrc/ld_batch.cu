@@ -73,9 +73,10 @@ constexpr int QSLOTS = 4;                                    // item ring depth
 // unpack and epilogue warps; rank 1's TMA thread, unpack and epilogue warps
 // Epilogue warps per r^2 mode: eight in R2_EXACT, twelve in R2_REFERENCE,
 // whose longer per-pair sequence leaves items below ~6,000 samples waiting
-// on their epilogue (4,096-task mix, reference mode: 87.7 against 95.0 ms;
-// exact mode with twelve: 72.1 against 69.2 ms, its 32-column chunks spill
-// at the 80 registers 704 threads leave).
+// on their epilogue (300-task mix, reference mode: 689 us against 706 with
+// eight; exact mode with twelve: 574 against 566, at the 80 registers 704
+// threads leave).  Popping the next item early to prefetch its factors, as
+// ld_mxf4_pair.cu does for its fixed tile list, costs 3 % here: 584.
 template <int MODE>
 struct Roles {
     static constexpr int EPI_WARPS = MODE == R2_REFERENCE ? 12 : 8;
@@ -389,15 +390,16 @@ k_ld_batch(const BatchParams bp) {
             if (*epi_fail || it.job < 0) break;
             const BatchJob &J = bp.jobs[it.job];
             const int ab = qi & 1;
+            bool special = false;
             if (et < COLS_N) {   // every column factor the chunks read; 0 past the tile and the task
                 const int b = it.tb * BN + et;
                 const uint32_t cb = (et < BN && b < J.n) ? J.bcB[b] : 0u;
                 if constexpr (MODE == R2_EXACT)
-                    epi::store_col_f32(colsf, et, cb, J.S);
+                    special = epi::store_col_f32(colsf, et, cb, J.S);
                 else
                     epi::store_col_ref(colsr, et, cb, J.S);
             }
-            named_bar_sync(1, R::EPI_THREADS);
+            const bool cols_special = named_bar_or(1, R::EPI_THREADS, special);
             bool ready = mbar_wait(smem_u32(&accfull[ab]), (qi >> 1) & 1, limit, bp.status);
             ready = __all_sync(0xffffffffu, ready);
             if (!ready) {
@@ -415,22 +417,19 @@ k_ld_batch(const BatchParams bp) {
                 const epi::ARowF raf = epi::make_arow_f32(ca, J.S);
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                // columns of the last 32-column chunk past the tile's 240 B rows
-                // are read but not written
                 const int n_tile = it.tb * BN + BN < J.n ? it.tb * BN + BN : J.n;
                 const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
                 epi::SumAcc acc;
-                // chunks of CW columns: 32 in exact mode; 16 in reference mode, whose
-                // longer epilogue runs faster on fewer live registers (182 against
-                // 199 ms on the 4,096-task mix; exact mode: 70.5 against 71.7 ms)
-                constexpr int CW = MODE == R2_EXACT ? 32 : 16;
+                // 16-column chunks, the tile's 15 (with 32 columns the exact mode's
+                // packed arithmetic spills: 620 against 566 us on 300 tasks)
+                constexpr int CW = 16;
 #pragma unroll 1
-                for (int c = colh; c < (BN + CW - 1) / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
+                for (int c = colh; c < BN / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
                     uint32_t v[CW];
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, c * CW,
+                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special, c * CW,
                                            it.tb * BN + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
                                            J.ldr, J.counts, J.ldc, 0, J.S);
                         if (J.summary)

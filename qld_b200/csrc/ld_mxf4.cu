@@ -312,15 +312,16 @@ k_ld_mxf4(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
             tl.decode_from(tile, ta, tb, cur_t, cur_base);
             const int lim = (it + 1) * nu + UST;
             produce_until(lim < total_u ? lim : total_u);
+            bool special = false;
             if (wt < COLS_N) {   // every column factor the chunks read; 0 past the tile
                 const int b = tb * BN + wt;
                 const uint32_t cb = (wt < BN && b < p.n) ? p.bcB[b] : 0u;
                 if constexpr (MODE == R2_EXACT)
-                    epi::store_col_f32(colsf, wt, cb, p.S);
+                    special = epi::store_col_f32(colsf, wt, cb, p.S);
                 else
                     epi::store_col_ref(colsr, wt, cb, p.S);
             }
-            named_bar_sync(1, WORKERS);
+            const bool cols_special = named_bar_or(1, WORKERS, special);
             bool ready = ok && !failed && mbar_wait(smem_u32(accfull), it & 1, p.timeout_cycles,
                                                     p.status);
             ready = __all_sync(0xffffffffu, ready);
@@ -340,15 +341,17 @@ k_ld_mxf4(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUten
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)acc_i * ACC1;
                 // columns past the tile's 240 B rows are read but not written
                 const int n_tile = tb * BN + BN < p.n ? tb * BN + BN : p.n;
+                // exact mode in 16-column chunks (32 columns' packed arithmetic spills)
+                constexpr int CW = MODE == R2_EXACT ? 16 : 32;
 #pragma unroll 1
-                for (int c = colh; c < 8; c += 2) {
-                    uint32_t v[32];
+                for (int c = colh; c < 256 / CW; c += 2) {
+                    uint32_t v[CW];
                     __syncwarp();
-                    tc_ld_32x32b_x32(tbase + (uint32_t)(c * 32), v);
+                    tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32(v, tbase + (uint32_t)(c * 32), raf, colsf, c * 32,
-                                       tb * BN + c * 32, a, a_ok, n_tile,
-                                       dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
+                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
+                                           c * CW, tb * BN + c * CW, a, a_ok, n_tile, dlo, dhi,
+                                           p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
                     } else {
                         // the F32 accumulators hold the counts as floats
                         epi::chunk_ref<0, true>(v, ra, colsr, c * 32, tb * BN + c * 32, a, a_ok,

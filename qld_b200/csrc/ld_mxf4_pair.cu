@@ -41,6 +41,11 @@
 //                accumulator buffer the tile used, every other one of its
 //                fifteen 16-column chunks, applies the r^2 epilogue (gemm_cpu.c:343-404) and
 //                stores; they arrive on rank 0's "accumulator empty" barrier.
+//                The next tile's bit counts load meanwhile: loading them and
+//                dividing at the tile's start cost 2,600-4,600 of the 12,000-
+//                23,000 cycles a tile's epilogue took.  Twelve epilogue warps
+//                (80 registers): band of 1,000 210 us against 199, reference
+//                mode 347 against 341.
 // Every wait is bounded.  No thread returns early: both CTAs meet at the
 // cluster barriers at start and end on every path, including after a
 // timeout, and the TMEM is released only after the last MMA has completed.
@@ -64,7 +69,7 @@ constexpr int SUB = 2;                   // unpacked stages (256 samples) per pa
 constexpr int UST = 4;                   // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;    // 8 KB
 constexpr int P_TX = (HM + HN) * PW * 8; // 15.5 KB delivered per stage
-constexpr int P_BYTES = 16384;           // stage stride: A rows, then B rows
+constexpr int P_BYTES = 15872;           // stage stride: A rows, then B rows (a multiple of 512)
 constexpr int UA_BYTES = HM * 128;       // 16 KB: 256 E2M1 per row
 constexpr int U_BYTES = (HM + HN) * 128; // 31 KB: A rows, then B rows
 constexpr int GROUPS = 4, GROUP_WARPS = 2;
@@ -95,21 +100,20 @@ struct Smem {
     static constexpr int OFF_P = OFF_U + UST * U_BYTES;
     static constexpr int OFF_ROWS = OFF_P + PST * P_BYTES;
     static constexpr int ROWS_BYTES = COLS_N * (MODE == R2_EXACT ? 8 : epi::COLR_BYTES);
-    static constexpr int OFF_BAR = OFF_ROWS + ROWS_BYTES;
+    static constexpr int OFF_BAR = OFF_ROWS + 2 * ROWS_BYTES;   // this tile's and the next one's
     static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1;
     static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
     static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
-                      P_TX <= P_BYTES,
-                  "swizzled stages must start on 1024-byte boundaries");
+                      P_BYTES % 512 == 0 && P_TX <= P_BYTES,
+                  "swizzled stages must start on whole swizzle atoms");
     // a group sees every (GROUPS / 2)-th packed stage or so: a slot must
     // always belong to the same groups for its phase bit to be enough
     static_assert(PST * SUB % GROUPS == 0 && GROUPS <= UST, "stage rings");
 };
-static_assert(sizeof(float2) == 8, "ColsF entry");
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
-static_assert(SUB == 2 && EPILOGUE == COLS_N, "work split");
+static_assert(SUB == 2 && EPILOGUE >= COLS_N && EPI_WARPS % 4 == 0, "work split");
 
 // BAND: a band's launch (its window and tiles); otherwise two regions or a
 // single region.  One kernel for both ran the other two 1.2 % slower.
@@ -129,8 +133,6 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint64_t *accempty = accfull + 2;
     uint64_t *mma_done = accempty + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM);
-    const epi::ColsR colsr(smem + L::OFF_ROWS, COLS_N);   // R2_REFERENCE factors
-    const epi::ColsF colsf(smem + L::OFF_ROWS, COLS_N);   // R2_EXACT: FP32 factors
 
     const uint32_t rank = cluster_rank();
     const int pair = (int)cluster_id_x(), npairs = (int)cluster_count_x();
@@ -291,25 +293,46 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else {
         // ------------------------------------------------------- epilogue --
+        // The bit counts of the next tile's rows are loaded while this tile is
+        // worked on, and its factors stored in the other half of the buffer.
         const int et = tid - FIRST_EPI_WARP * 32;
         const int ew = warp - FIRST_EPI_WARP;
         const int q = warp & 3;                 // TMEM lane quarter
-        const int colh = ew >> 2;               // chunks colh, colh + 2, ... (< 15)
+        const int colh = ew >> 2;               // chunks colh, colh + EPI_WARPS / 4, ... (< 15)
         bool failed = false;
-        int cur_t = 0, cur_base = 0;
-        for (int it = 0; it < my_tiles; ++it) {
-            int a_row, b_row;
+        int cur_t = 0, cur_base = 0, a_row = 0, b_row = 0;
+        uint32_t ca = 0, cb = 0;                // bit counts of my row and column
+        auto load_counts = [&](int it) {
             tl.decode_from(pair + it * npairs, a_row, b_row, cur_t, cur_base);
-            const int ab = it & 1;
-            {   // every column factor the chunks read; 0 past the tile and the task
-                const int b = b_row + et;
-                const uint32_t cb = (et < BN && b < p.n) ? p.bcB[b] : 0u;
-                if constexpr (MODE == R2_EXACT)
-                    epi::store_col_f32(colsf, et, cb, p.S);
-                else
-                    epi::store_col_ref(colsr, et, cb, p.S);
+            const int a = a_row + (int)rank * HM + q * 32 + lane, b = b_row + et;
+            ca = a < p.m ? p.bcA[a] : 0u;
+            // every column factor the chunks read; 0 past the tile and the task
+            cb = et < BN && b < p.n ? p.bcB[b] : 0u;
+        };
+        epi::ARowR ra{};
+        epi::ARowF raf{};
+        bool special = false;
+        auto store_factors = [&](int it) {
+            uint8_t *base = smem + L::OFF_ROWS + (it & 1) * L::ROWS_BYTES;
+            if constexpr (MODE == R2_EXACT) {
+                raf = epi::make_arow_f32(ca, p.S);
+                special = et < COLS_N && epi::store_col_f32(epi::ColsF(base, COLS_N), et, cb, p.S);
+            } else {
+                ra = epi::make_arow_ref(ca, p.S);
+                if (et < COLS_N) epi::store_col_ref(epi::ColsR(base, COLS_N), et, cb, p.S);
             }
-            named_bar_sync(1, EPILOGUE);
+        };
+        if (my_tiles > 0) {
+            load_counts(0);
+            store_factors(0);
+        }
+        for (int it = 0; it < my_tiles; ++it) {
+            const int ab = it & 1;
+            const int a = a_row + (int)rank * HM + q * 32 + lane, b_tile = b_row;
+            const bool a_ok = a < p.m;
+            // this tile's factors are stored, and the other half is free
+            const bool cols_special = named_bar_or(1, EPILOGUE, special);
+            if (it + 1 < my_tiles) load_counts(it + 1);
             bool ready = !failed && mbar_wait(smem_u32(&accfull[ab]), (it >> 1) & 1,
                                               p.timeout_cycles, p.status);
             ready = __all_sync(0xffffffffu, ready);
@@ -320,37 +343,35 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (ready) {
                 __syncwarp();
                 tc_fence_after();
-                const int a = a_row + (int)rank * HM + q * 32 + lane;
-                const bool a_ok = a < p.m;
-                const uint32_t ca = a_ok ? p.bcA[a] : 0u;
-                const epi::ARowR ra = epi::make_arow_ref(ca, p.S);
-                const epi::ARowF raf = epi::make_arow_f32(ca, p.S);
+                uint8_t *base = smem + L::OFF_ROWS + ab * L::ROWS_BYTES;
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                const int n_tile = b_row + BN < p.n ? b_row + BN : p.n;
+                const int n_tile = b_tile + BN < p.n ? b_tile + BN : p.n;
                 // 16-column chunks: fewer live registers than 32 (2.41 / 2.66 ms
                 // against 2.43 / 2.75 ms, exact / reference r^2), the tile's 15
 #pragma unroll 1
-                for (int c = colh; c < BN / 16; c += 2) {
+                for (int c = colh; c < BN / 16; c += EPI_WARPS / 4) {
                     uint32_t v[16];
                     __syncwarp();
                     tc_ld_32x32b_x16(tbase + (uint32_t)(c * 16), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<16>(v, tbase + (uint32_t)(c * 16), raf, colsf, c * 16,
-                                           b_row + c * 16, a, a_ok, n_tile,
-                                           dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
+                        epi::chunk_f32<16>(v, tbase + (uint32_t)(c * 16), raf,
+                                           epi::ColsF(base, COLS_N), cols_special, c * 16,
+                                           b_tile + c * 16, a, a_ok, n_tile, dlo, dhi, p.r2, p.ldr,
+                                           p.counts, p.ldc, p.out_row0, p.S);
                     } else {
                         // the F32 accumulators hold the counts as floats
-                        epi::chunk_ref<0, true, 16>(v, ra, colsr, c * 16, b_row + c * 16, a, a_ok,
-                                            n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc,
-                                            p.out_row0, p.S);
+                        epi::chunk_ref<0, true, 16>(v, ra, epi::ColsR(base, COLS_N), c * 16,
+                                                    b_tile + c * 16, a, a_ok, n_tile, dlo, dhi,
+                                                    p.r2, p.ldr, p.counts, p.ldc, p.out_row0,
+                                                    p.S);
                     }
                 }
                 tc_fence_before();
                 __syncwarp();
                 if (lane == 0) mbar_arrive_rank(smem_u32(&accempty[ab]), 0);
             }
-            named_bar_sync(1, EPILOGUE);
+            if (it + 1 < my_tiles) store_factors(it + 1);
         }
     }
 

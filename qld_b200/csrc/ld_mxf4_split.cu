@@ -165,7 +165,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     const uint32_t tbase = tmem + ((uint32_t)(q * 32) << 16);
     epi::ARowR ra{};
     epi::ARowF raf{};
-    bool ready = false;
+    bool ready = false, cols_special = false;
 
     if (warp == 0) {
         // ------------------------------------------------------- producer --
@@ -226,10 +226,11 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     } else {
         // --------------------------------------------------------- unpack --
         const int wt = tid - FIRST_WORKER * 32;
+        bool special = false;
         if (wt < bn) {
             const int b = b_row + wt;
             const uint32_t cb = b < p.n ? p.bcB[b] : 0u;
-            if constexpr (MODE == R2_EXACT) epi::store_col_f32(colsf, wt, cb, p.S);
+            if constexpr (MODE == R2_EXACT) special = epi::store_col_f32(colsf, wt, cb, p.S);
             else epi::store_col_ref(colsr, wt, cb, p.S);
         }
         const uint32_t ca = a_ok ? p.bcA[a] : 0u;
@@ -267,7 +268,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 mbar_arrive(smem_u32(&pempty[ps]));
             }
         }
-        named_bar_sync(1, WORKERS);                // the column factors are stored
+        cols_special = named_bar_or(1, WORKERS, special);   // the column factors are stored
         // the accumulators; on a failed wait the drain wait still keeps the
         // CTA until its MMAs are done
         ready = mbar_wait(smem_u32(accfull), 0, ok ? p.timeout_cycles : 1, p.status);
@@ -318,8 +319,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                 if constexpr (MODE == R2_EXACT) tc_st_32x32b_x16(taddr, v);
             }
             if constexpr (MODE == R2_EXACT)
-                epi::chunk_f32<CH>(v, taddr, raf, colsf, c * CH, b_row + c * CH, a, a_ok, n_tile,
-                                   dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
+                epi::chunk_f32<CH>(v, taddr, raf, colsf, cols_special, c * CH, b_row + c * CH, a,
+                                   a_ok, n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
             else
                 epi::chunk_ref<0, true, CH>(v, ra, colsr, c * CH, b_row + c * CH, a, a_ok, n_tile,
                                             dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0,

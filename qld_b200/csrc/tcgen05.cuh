@@ -329,6 +329,20 @@ __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
+// named_bar_sync that also tells every thread whether `x` held in any of them.
+__device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool x) {
+    uint32_t r;
+    asm volatile(
+        "{\n\t.reg .pred p, q;\n\t"
+        "setp.ne.u32 p, %3, 0;\n\t"
+        "bar.red.or.pred q, %1, %2, p;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(r)
+        : "r"(id), "r"(nthreads), "r"((uint32_t)x)
+        : "memory");
+    return r != 0u;
+}
+
 __device__ __forceinline__ uint32_t imul(uint32_t a, uint32_t b) {
     uint32_t r;
     asm("mul.lo.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
