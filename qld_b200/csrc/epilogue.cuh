@@ -79,10 +79,39 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 // a test.  A row with v >= 1 (c = S, or a bit count above S) carries a NaN
 // in y, which sends every pair with it to the literal sequence.
 struct ColsR {
+    static constexpr bool PAIRS = false;
     float4 *f;
     __device__ __forceinline__ ColsR(uint8_t *base, int) : f(reinterpret_cast<float4 *>(base)) {}
+    __device__ __forceinline__ float4 col(int bl) const { return f[bl]; }
+    __device__ __forceinline__ void put(int bl, float4 k) const { f[bl] = k; }
 };
 constexpr int COLR_BYTES = 16;
+
+// The same factors by column pairs, each of the four as an f2: x, y, z, w.
+struct ColsR2 {
+    static constexpr bool PAIRS = true;
+    float *f;
+    __device__ __forceinline__ ColsR2(uint8_t *base, int) : f(reinterpret_cast<float *>(base)) {}
+    __device__ __forceinline__ float4 col(int bl) const {
+        const float *p = f + (bl >> 1) * 8 + (bl & 1);
+        return make_float4(p[0], p[2], p[4], p[6]);
+    }
+    __device__ __forceinline__ void put(int bl, float4 k) const {
+        float *p = f + (bl >> 1) * 8 + (bl & 1);
+        p[0] = k.x;
+        p[2] = k.y;
+        p[4] = k.z;
+        p[6] = k.w;
+    }
+    __device__ __forceinline__ void pair(int bl, f2 &x, f2 &y, f2 &z, f2 &w) const {   // bl even
+        const ulonglong2 a = *reinterpret_cast<const ulonglong2 *>(f + bl * 4);
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2 *>(f + bl * 4 + 4);
+        x = a.x;
+        y = a.y;
+        z = b.x;
+        w = b.y;
+    }
+};
 
 __device__ __forceinline__ float4 ref_factors(uint32_t c, int S) {
     if (c == 0u) return make_float4(0.0f, 0.0f, 0.0f, 0.0f);
@@ -94,8 +123,9 @@ __device__ __forceinline__ float4 ref_factors(uint32_t c, int S) {
     return make_float4(v, hi, __double2float_rn(__dsub_rn(i, (double)hi)), __frcp_rn(v));
 }
 
-__device__ __forceinline__ void store_col_ref(const ColsR &f, int bl, uint32_t c, int S) {
-    f.f[bl] = ref_factors(c, S);
+template <class C>
+__device__ __forceinline__ void store_col_ref(const C &f, int bl, uint32_t c, int S) {
+    f.put(bl, ref_factors(c, S));
 }
 
 // Per-thread A-row factors of the reference mode.
@@ -112,6 +142,28 @@ __device__ __forceinline__ ARowR make_arow_ref(uint32_t c, int S) {
     r.Sf = (float)S;
     r.rSf = __frcp_rn(r.Sf);
     return r;
+}
+
+// Columns t of a chunk (B rows b0 + t, t < CW <= 32) that A row a owes: inside
+// the task (b < n) and the diagonal window dlo <= a - b <= dhi, as a bit mask.
+template <int CW>
+__device__ __forceinline__ uint32_t column_mask(int b0, int a, bool a_ok, int n, int dlo,
+                                                int dhi) {
+    int lo = 0, hi = n - b0 < CW ? n - b0 : CW;
+    if (dlo > -2147483647 - 1 && a - b0 - dlo + 1 < hi) hi = a - b0 - dlo + 1;
+    if (dhi < 2147483647 && a - b0 - dhi > 0) lo = a - b0 - dhi;
+    if (!a_ok || lo >= hi) return 0u;
+    return (0xFFFFFFFFu >> (32 - hi)) & (0xFFFFFFFFu << lo);
+}
+
+// *p = x if cond, as a predicated store: no branch, so the arithmetic around
+// it is scheduled across it.
+__device__ __forceinline__ void store_if(uint32_t *p, uint32_t x, bool cond) {
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "setp.ne.u32 q, %2, 0;\n\t"
+        "@q st.global.u32 [%0], %1;\n\t}" ::"l"(p),
+        "r"(x), "r"((uint32_t)cond));
 }
 
 // Shared-memory column factors of one tile for the integer-count kernels:
@@ -235,6 +287,46 @@ __device__ __forceinline__ float r2_reference_ff(float cab, const ARowR &A, floa
     return rh > __uint_as_float(0x3F800000u + 838u) ? 123.456f : rh;
 }
 
+// r2_reference_ff for two columns (f2 halves): the same operations with the
+// same roundings, a subtraction x - y written as an addition of -y computed
+// as (-a) * b.  Leaves q (before the > 1.0001 rule) and x, and sets a flag
+// per half as r2_reference_ff's `redo`.
+struct ARowR2 {
+    f2 rS, nS, v, nv, y, ny, z, w;
+    __device__ __forceinline__ explicit ARowR2(const ARowR &a)
+        : rS(splat2(a.rSf)), nS(splat2(-a.Sf)), v(splat2(a.k.x)), nv(splat2(-a.k.x)),
+          y(splat2(a.k.y)), ny(splat2(-a.k.y)), z(splat2(a.k.z)), w(splat2(a.k.w)) {}
+};
+
+__device__ __forceinline__ void r2_reference_ff2(f2 cab, const ARowR2 &A, f2 bx, f2 by, f2 bz,
+                                                 f2 bw, float &q0, float &q1, bool &redo0,
+                                                 bool &redo1) {
+    f2 v3 = mul2(cab, A.rS);
+    v3 = fma2(fma2(v3, A.nS, cab), A.rS, v3);
+    const f2 np12 = mul2(A.nv, bx);
+    const f2 e = fma2(A.v, bx, np12);
+    const f2 d = add2(v3, np12);
+    const f2 x = mul2(d, d);
+    const f2 nPh = mul2(A.ny, by), Ph = mul2(A.y, by);
+    f2 Pl = fma2(A.y, by, nPh);
+    Pl = fma2(A.y, bz, Pl);
+    Pl = fma2(A.z, by, Pl);
+    const f2 t = mul2(e, mul2(A.w, bw));
+    const f2 qh = mul2(x, Ph);
+    f2 ql = fma2(x, Ph, mul2(x, nPh));
+    ql = fma2(x, Pl, ql);
+    ql = fma2(qh, t, ql);
+    const f2 rh = add2(qh, fma2(qh, splat2(0x1p-40f), ql));
+    const f2 rl = add2(qh, fma2(qh, splat2(-0x1p-40f), ql));
+    float l0, l1, x0, x1;
+    unpack2(rh, q0, q1);
+    unpack2(rl, l0, l1);
+    unpack2(x, x0, x1);
+    const uint32_t tiny = __float_as_uint(0x1p-100f) - 1u;
+    redo0 = !(q0 == l0) || __float_as_uint(x0) - 1u < tiny;
+    redo1 = !(q1 == l1) || __float_as_uint(x1) - 1u < tiny;
+}
+
 // A pair the fast path flagged.  A fixed SNP (v = 1: every sample carries
 // the allele) makes the reference's denominator p12 (1 - vA)(1 - vB) exactly
 // +0, so its quotient is x / +0 = +inf, hence 123.456, or 0 / 0, the x86
@@ -254,39 +346,82 @@ __device__ __forceinline__ float r2_flagged(uint32_t cab, const RowRef &A, const
     return r2_reference(cab, A, B, S);
 }
 
-// The reference-mode chunk of CW (<= 32) columns: every pair on the fast
-// path, the flagged ones (their accumulator word kept in v, a bit in `redo`)
-// redone with r2_flagged.
-// FLOATCNT: v holds each count as F32 bits (the 4-bit kernels' accumulators),
-// else as an integer shifted left by SHIFT.
-template <int SHIFT, bool FLOATCNT, int CW = 32>
-__device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, const ColsR &f,
-                                          int bl0, int b0, int a, bool a_ok, int n, int dlo,
-                                          int dhi, float *r2, long long ldr, uint32_t *counts,
-                                          long long ldc, int row0, int S) {
-    uint32_t *oc = (counts && a_ok) ? counts + (long long)(b0 - row0) * ldc + a : nullptr;
+// The fast path over a reference-mode chunk: v becomes the results, a flagged
+// pair keeps its accumulator word; returns the flagged columns.  put(t, c)
+// takes every column's count: interleaved with the arithmetic, as its stores
+// would otherwise queue up before it.
+template <int SHIFT, bool FLOATCNT, int CW, class C, class Put>
+__device__ __forceinline__ uint32_t ref_columns(uint32_t (&v)[CW], const ARowR &ra, const C &f,
+                                                int bl0, int S, Put put) {
+    auto count = [&](int t) {
+        return FLOATCNT ? (uint32_t)__uint_as_float(v[t]) : v[t] >> SHIFT;
+    };
     uint32_t redo = 0;
-    if (S <= (1 << 24)) {
+    if (S > (1 << 24)) {
 #pragma unroll
-        for (int t = 0; t < CW; ++t) {
-            const uint32_t raw = v[t];
-            const float cf = FLOATCNT ? __uint_as_float(raw) : (float)(raw >> SHIFT);
-            const int b = b0 + t;
-            if (oc && b < n && a - b >= dlo && a - b <= dhi)
-                oc[(long long)t * ldc] = FLOATCNT ? (uint32_t)cf : raw >> SHIFT;
-            bool rd;
-            const float r = r2_reference_ff(cf, ra, f.f[bl0 + t], rd);
-            v[t] = rd ? raw : __float_as_uint(r);   // a flagged pair keeps its count
-            redo |= (uint32_t)rd << t;
+        for (int t = 0; t < CW; ++t) put(t, count(t));
+        redo = CW == 32 ? 0xFFFFFFFFu : (1u << CW) - 1u;
+    } else if constexpr (C::PAIRS) {
+        const ARowR2 A(ra);
+        float rmax = 0.0f;
+#pragma unroll
+        for (int t = 0; t < CW; t += 2) {
+            put(t, count(t));
+            put(t + 1, count(t + 1));
+            f2 bx, by, bz, bw;
+            f.pair(bl0 + t, bx, by, bz, bw);
+            float q0, q1;
+            bool rd0, rd1;
+            r2_reference_ff2(pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1])), A, bx, by,
+                             bz, bw, q0, q1, rd0, rd1);
+            rmax = max3(rmax, q0, q1);
+            v[t] = rd0 ? v[t] : __float_as_uint(q0);
+            v[t + 1] = rd1 ? v[t + 1] : __float_as_uint(q1);
+            redo |= (uint32_t)rd0 << t | (uint32_t)rd1 << (t + 1);
+        }
+        const float limit = __uint_as_float(0x3F800000u + 838u);
+        if (__any_sync(0xffffffffu, rmax > limit)) {
+#pragma unroll
+            for (int t = 0; t < CW; ++t)
+                if (!((redo >> t) & 1u) && __uint_as_float(v[t]) > limit)
+                    v[t] = __float_as_uint(123.456f);
         }
     } else {
 #pragma unroll
         for (int t = 0; t < CW; ++t) {
-            const uint32_t cnt = FLOATCNT ? (uint32_t)__uint_as_float(v[t]) : v[t] >> SHIFT;
-            const int b = b0 + t;
-            if (oc && b < n && a - b >= dlo && a - b <= dhi) oc[(long long)t * ldc] = cnt;
+            const uint32_t raw = v[t];
+            put(t, count(t));
+            bool rd;
+            const float r = r2_reference_ff(FLOATCNT ? __uint_as_float(raw) : (float)(raw >> SHIFT),
+                                            ra, f.col(bl0 + t), rd);
+            v[t] = rd ? raw : __float_as_uint(r);
+            redo |= (uint32_t)rd << t;
         }
-        redo = CW == 32 ? 0xFFFFFFFFu : (1u << CW) - 1u;
+    }
+    return redo;
+}
+
+// The reference-mode chunk of CW (<= 32) columns: every pair on the fast
+// path, the flagged ones (their accumulator word kept in v, a bit in `redo`)
+// redone with r2_flagged.
+// FLOATCNT: v holds each count as F32 bits (the 4-bit kernels' accumulators),
+// else as an integer shifted left by SHIFT.  With ColsR2 the fast path runs on
+// two columns at a time (FLOATCNT only).
+template <int SHIFT, bool FLOATCNT, int CW = 32, class C>
+__device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, const C &f,
+                                          int bl0, int b0, int a, bool a_ok, int n, int dlo,
+                                          int dhi, float *r2, long long ldr, uint32_t *counts,
+                                          long long ldc, int row0, int S) {
+    static_assert(FLOATCNT || !C::PAIRS, "packed pairs take F32 counts");
+    uint32_t redo = 0;
+    if (counts) {
+        uint32_t *oc = counts + (long long)(b0 - row0) * ldc + a;
+        const uint32_t mask = column_mask<CW>(b0, a, a_ok, n, dlo, dhi);
+        redo = ref_columns<SHIFT, FLOATCNT, CW>(v, ra, f, bl0, S, [&](int t, uint32_t c) {
+            store_if(oc + (long long)t * ldc, c, (mask >> t) & 1u);
+        });
+    } else {
+        redo = ref_columns<SHIFT, FLOATCNT, CW>(v, ra, f, bl0, S, [](int, uint32_t) {});
     }
     if (!a_ok) redo = 0;
     if (__any_sync(0xffffffffu, redo != 0)) {
@@ -298,7 +433,7 @@ __device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, co
         if (__any_sync(0xffffffffu, a_fixed) && a_fixed) {
 #pragma unroll
             for (int t = 0; t < CW; ++t) {
-                const float vb = f.f[bl0 + t].x;
+                const float vb = f.col(bl0 + t).x;
                 if (((redo >> t) & 1u) && vb <= 1.0f) {
                     const float cf = FLOATCNT ? __uint_as_float(v[t]) : (float)(v[t] >> SHIFT);
                     v[t] = __float_as_uint(
@@ -316,7 +451,7 @@ __device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, co
             for (int t = 0; t < CW; ++t) {
                 const bool rd = (redo >> t) & 1u;
                 if (__any_sync(0xffffffffu, rd) && rd) {
-                    const float4 cb = f.f[bl0 + t];
+                    const float4 cb = f.col(bl0 + t);
                     RowRef rb;
                     rb.c = cb.x != 0.0f;        // only the zero rule reads it
                     rb.v = cb.x;

@@ -73,8 +73,8 @@ constexpr int QSLOTS = 4;                                    // item ring depth
 // unpack and epilogue warps; rank 1's TMA thread, unpack and epilogue warps
 // Epilogue warps per r^2 mode: eight in R2_EXACT, twelve in R2_REFERENCE,
 // whose longer per-pair sequence leaves items below ~6,000 samples waiting
-// on their epilogue (300-task mix, reference mode: 689 us against 706 with
-// eight; exact mode with twelve: 574 against 566, at the 80 registers 704
+// on their epilogue (300-task mix, one-column arithmetic: 689 us against 706
+// with eight; exact mode with twelve: 574 against 566, at the 80 registers 704
 // threads leave).  Popping the next item early to prefetch its factors, as
 // ld_mxf4_pair.cu does for its fixed tile list, costs 3 % here: 584.
 template <int MODE>
@@ -153,7 +153,7 @@ k_ld_batch(const BatchParams bp) {
     uint64_t *ifull = mma_done + 1, *iempty = ifull + QSLOTS;
     Item *items = reinterpret_cast<Item *>(smem + L::OFF_ITEMS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM);
-    const epi::ColsR colsr(smem + L::OFF_ROWS, COLS_N);   // R2_REFERENCE factors
+    const epi::ColsR2 colsr(smem + L::OFF_ROWS, COLS_N);   // R2_REFERENCE factors
     const epi::ColsF colsf(smem + L::OFF_ROWS, COLS_N);   // R2_EXACT: FP32 factors
 
     const uint32_t rank = cluster_rank();
@@ -420,9 +420,10 @@ k_ld_batch(const BatchParams bp) {
                 const int n_tile = it.tb * BN + BN < J.n ? it.tb * BN + BN : J.n;
                 const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
                 epi::SumAcc acc;
-                // 16-column chunks, the tile's 15 (with 32 columns the exact mode's
-                // packed arithmetic spills: 620 against 566 us on 300 tasks)
-                constexpr int CW = 16;
+                // Chunks of 16 columns, in reference mode of 8 (more columns spill:
+                // 32 in exact mode 620 us against 566 on 300 tasks, 16 in
+                // reference mode 668 against 647)
+                constexpr int CW = MODE == R2_EXACT ? 16 : 8;
 #pragma unroll 1
                 for (int c = colh; c < BN / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
                     uint32_t v[CW];

@@ -319,7 +319,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 special = et < COLS_N && epi::store_col_f32(epi::ColsF(base, COLS_N), et, cb, p.S);
             } else {
                 ra = epi::make_arow_ref(ca, p.S);
-                if (et < COLS_N) epi::store_col_ref(epi::ColsR(base, COLS_N), et, cb, p.S);
+                if (et < COLS_N) epi::store_col_ref(epi::ColsR2(base, COLS_N), et, cb, p.S);
             }
         };
         if (my_tiles > 0) {
@@ -347,22 +347,24 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
                 const int n_tile = b_tile + BN < p.n ? b_tile + BN : p.n;
-                // 16-column chunks: fewer live registers than 32 (2.41 / 2.66 ms
-                // against 2.43 / 2.75 ms, exact / reference r^2), the tile's 15
+                // Chunks of 16 columns, in reference mode of 8: their packed
+                // arithmetic keeps more values live (16 columns spill: band of
+                // 1,000 in reference mode 244 us against 241).
+                constexpr int CW = MODE == R2_EXACT ? 16 : 8;
 #pragma unroll 1
-                for (int c = colh; c < BN / 16; c += EPI_WARPS / 4) {
-                    uint32_t v[16];
+                for (int c = colh; c < BN / CW; c += EPI_WARPS / 4) {
+                    uint32_t v[CW];
                     __syncwarp();
-                    tc_ld_32x32b_x16(tbase + (uint32_t)(c * 16), v);
+                    tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<16>(v, tbase + (uint32_t)(c * 16), raf,
-                                           epi::ColsF(base, COLS_N), cols_special, c * 16,
-                                           b_tile + c * 16, a, a_ok, n_tile, dlo, dhi, p.r2, p.ldr,
+                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf,
+                                           epi::ColsF(base, COLS_N), cols_special, c * CW,
+                                           b_tile + c * CW, a, a_ok, n_tile, dlo, dhi, p.r2, p.ldr,
                                            p.counts, p.ldc, p.out_row0, p.S);
                     } else {
                         // the F32 accumulators hold the counts as floats
-                        epi::chunk_ref<0, true, 16>(v, ra, epi::ColsR(base, COLS_N), c * 16,
-                                                    b_tile + c * 16, a, a_ok, n_tile, dlo, dhi,
+                        epi::chunk_ref<0, true, CW>(v, ra, epi::ColsR2(base, COLS_N), c * CW,
+                                                    b_tile + c * CW, a, a_ok, n_tile, dlo, dhi,
                                                     p.r2, p.ldr, p.counts, p.ldc, p.out_row0,
                                                     p.S);
                     }

@@ -112,7 +112,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
     uint64_t *ufull = pempty + MAX_PST, *uempty = ufull + UST;
     uint64_t *accfull = uempty + UST;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L.bars + NBARS * 8);
-    const epi::ColsR colsr(smem + L.cols, MAX_BN);
+    const epi::ColsR2 colsr(smem + L.cols, MAX_BN);
     const epi::ColsF colsf(smem + L.cols, MAX_BN);
 
     const uint32_t crank = cluster_rank();
@@ -304,27 +304,35 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
 #pragma unroll 1
         for (int i = cg; i * ks + split < chunks; i += 4) {
             const int c = i * ks + split;
-            const uint32_t taddr = tbase + (uint32_t)(c * CH);
-            uint32_t v[CH];
-            __syncwarp();
-            tc_ld_32x32b_x16(taddr, v);
-            if (ks > 1) {
-                for (int o = 0; o < ks - 1; ++o) {
-                    const float *part = push + (o * per + i) * (SLOT_BYTES / 4) + q * 32 + lane;
+            // in reference mode in halves, whose packed arithmetic does not spill
+            constexpr int CW = MODE == R2_EXACT ? CH : CH / 2;
+#pragma unroll 1
+            for (int h = 0; h < CH; h += CW) {
+                const int col = c * CH + h;
+                const uint32_t taddr = tbase + (uint32_t)col;
+                uint32_t v[CW];
+                __syncwarp();
+                tc_ld_32x32b<CW>(taddr, v);
+                if (ks > 1) {
+                    for (int o = 0; o < ks - 1; ++o) {
+                        const float *part = push + (o * per + i) * (SLOT_BYTES / 4) + h * HM +
+                                            q * 32 + lane;
 #pragma unroll
-                    for (int t = 0; t < CH; ++t)
-                        v[t] = __float_as_uint(__uint_as_float(v[t]) + part[t * HM]);
+                        for (int t = 0; t < CW; ++t)
+                            v[t] = __float_as_uint(__uint_as_float(v[t]) + part[t * HM]);
+                    }
+                    // chunk_f32 re-reads the rare count it evaluates again
+                    if constexpr (MODE == R2_EXACT) tc_st_32x32b_x16(taddr, v);
                 }
-                // chunk_f32 re-reads the rare count it evaluates again
-                if constexpr (MODE == R2_EXACT) tc_st_32x32b_x16(taddr, v);
+                if constexpr (MODE == R2_EXACT)
+                    epi::chunk_f32<CW>(v, taddr, raf, colsf, cols_special, col, b_row + col, a,
+                                       a_ok, n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc,
+                                       p.out_row0, p.S);
+                else
+                    epi::chunk_ref<0, true, CW>(v, ra, colsr, col, b_row + col, a, a_ok, n_tile,
+                                                dlo, dhi, p.r2, p.ldr, p.counts, p.ldc,
+                                                p.out_row0, p.S);
             }
-            if constexpr (MODE == R2_EXACT)
-                epi::chunk_f32<CH>(v, taddr, raf, colsf, cols_special, c * CH, b_row + c * CH, a,
-                                   a_ok, n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0, p.S);
-            else
-                epi::chunk_ref<0, true, CH>(v, ra, colsr, c * CH, b_row + c * CH, a, a_ok, n_tile,
-                                            dlo, dhi, p.r2, p.ldr, p.counts, p.ldc, p.out_row0,
-                                            p.S);
         }
     }
 

@@ -317,11 +317,21 @@ __device__ __forceinline__ void tc_ld_32x32b_x16(uint32_t taddr, uint32_t (&v)[1
     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
 
-// 16 or 32 consecutive TMEM columns of the warp's lane quarter.
+__device__ __forceinline__ void tc_ld_32x32b_x8(uint32_t taddr, uint32_t (&v)[8]) {
+    asm volatile(
+        "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+          "=r"(v[7])
+        : "r"(taddr));
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+}
+
+// 8, 16 or 32 consecutive TMEM columns of the warp's lane quarter.
 template <int CW>
 __device__ __forceinline__ void tc_ld_32x32b(uint32_t taddr, uint32_t (&v)[CW]) {
-    static_assert(CW == 16 || CW == 32, "16 or 32 columns");
-    if constexpr (CW == 16) tc_ld_32x32b_x16(taddr, v);
+    static_assert(CW == 8 || CW == 16 || CW == 32, "8, 16 or 32 columns");
+    if constexpr (CW == 8) tc_ld_32x32b_x8(taddr, v);
+    else if constexpr (CW == 16) tc_ld_32x32b_x16(taddr, v);
     else tc_ld_32x32b_x32(taddr, v);
 }
 
