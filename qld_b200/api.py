@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes as ct
 import os
+import struct
 import weakref
 from dataclasses import dataclass
 
@@ -61,6 +62,12 @@ class _LdArgs(ct.Structure):
         ("r2", ct.c_void_p), ("ldr", ct.c_longlong),
         ("counts", ct.c_void_p), ("ldc", ct.c_longlong),
     ]
+
+
+# qld_ld_args as one native struct: packing a call's arguments costs about a
+# third of building the ctypes structure field by field.
+_LD_PACK = struct.Struct("@PPiqPPiqiiiPqPq")
+assert _LD_PACK.size == ct.sizeof(_LdArgs)
 
 
 class _Stats(ct.Structure):
@@ -153,6 +160,8 @@ def load_library(path: str = LIB_PATH) -> ct.CDLL:
     lib.qld_srv_destroy.argtypes = [vp]
     lib.qld_srv_last_error.argtypes = [vp]
     lib.qld_srv_last_error.restype = ct.c_char_p
+    # the device call again, taking its packed arguments as bytes
+    lib.ld_device_packed = ct.CFUNCTYPE(i, vp, ct.c_char_p, vp)(("qld_cuda_ld_device", lib))
     _lib = lib
     return lib
 
@@ -404,9 +413,11 @@ class Context:
     def ld_device(self, A, bcA, m, lda, B, bcB, n, ldb, K, S, symmetric, r2, ldr,
                   counts=None, ldc=0, stream=None):
         """Enqueue one task on device buffers (torch tensors or raw pointers)."""
-        a = _LdArgs(_p(A), _p(bcA), int(m), int(lda), _p(B), _p(bcB), int(n), int(ldb), int(K),
-                    int(S), int(bool(symmetric)), _p(r2), int(ldr), _p(counts), int(ldc))
-        self._check(self.lib.qld_cuda_ld_device(self.h, ct.byref(a), _stream(stream)))
+        rc = self.lib.ld_device_packed(
+            self.h, _pack_args(A, bcA, m, lda, B, bcB, n, ldb, K, S, symmetric, r2, ldr, counts,
+                               ldc), _stream(stream))
+        if rc != OK:
+            self._check(rc)
 
     def ld_device_part(self, A, bcA, m, lda, B, bcB, n, ldb, K, S, symmetric, r2, ldr, part,
                        nparts, counts=None, ldc=0, stream=None):
@@ -421,14 +432,17 @@ class Context:
 
     @staticmethod
     def _ld_args(jobs):
-        arr = (_LdArgs * len(jobs))()
-        for i, j in enumerate(jobs):
-            arr[i] = _LdArgs(_p(j["A"]), _p(j["bcA"]), int(j["m"]), int(j["lda"]),
-                             _p(j.get("B")), _p(j.get("bcB")), int(j.get("n", j["m"])),
-                             int(j.get("ldb", j["lda"])), int(j["K"]), int(j["S"]),
-                             int(bool(j["symmetric"])), _p(j["r2"]), int(j["ldr"]),
-                             _p(j.get("counts")), int(j.get("ldc", 0)))
-        return arr
+        size = _LD_PACK.size
+        buf = bytearray(size * len(jobs))
+        at = 0
+        for j in jobs:
+            get = j.get
+            m, lda = j["m"], j["lda"]
+            buf[at:at + size] = _pack_args(
+                j["A"], j["bcA"], m, lda, get("B"), get("bcB"), get("n", m), get("ldb", lda),
+                j["K"], j["S"], j["symmetric"], j["r2"], j["ldr"], get("counts"), get("ldc", 0))
+            at += size
+        return (_LdArgs * len(jobs)).from_buffer(buf)
 
     def ld_batch(self, jobs, stream=None):
         """Enqueue many tasks in one launch.  `jobs`: sequence of dicts with
@@ -523,6 +537,26 @@ def _p(x):
     if isinstance(x, int):
         return x
     return _ptr(x)
+
+
+def _addr(x) -> int:
+    """_p as an int (0 for None); torch tensors, the common case, first."""
+    try:
+        return x.data_ptr()
+    except AttributeError:
+        return _p(x) or 0
+
+
+def _pack_args(A, bcA, m, lda, B, bcB, n, ldb, K, S, symmetric, r2, ldr, counts, ldc) -> bytes:
+    """The bytes of a qld_ld_args."""
+    a = _addr(A), _addr(bcA), 0 if B is None else _addr(B), 0 if bcB is None else _addr(bcB)
+    out, cnt = _addr(r2), 0 if counts is None else _addr(counts)
+    try:
+        return _LD_PACK.pack(a[0], a[1], m, lda, a[2], a[3], n, ldb, K, S, bool(symmetric), out,
+                             ldr, cnt, ldc)
+    except struct.error:      # sizes that are not integers, or not of the field's width
+        return bytes(_LdArgs(a[0], a[1], int(m), int(lda), a[2], a[3], int(n), int(ldb), int(K),
+                             int(S), int(bool(symmetric)), out, int(ldr), cnt, int(ldc)))
 
 
 CUDA_STREAM_LEGACY = 1   # cudaStreamLegacy: the legacy default stream's handle
