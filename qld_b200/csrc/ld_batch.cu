@@ -8,33 +8,38 @@
 // fused r^2 epilogue of qLD gemm_cpu.c:343-404 (R2_EXACT in FP32 from the
 // exact counts, epilogue.cuh: chunk_f32).  qLD itself runs such task lists
 // one task at a time (-inputList, src/correlator/src/input_list.c:205-323
-// and correlate_function.c:59-83).  Here every 256 x 240 output tile of every
-// task is a work item, computed by a cluster of two CTAs (rank r: A rows
-// 128 r.., B rows 120 r.. of the tile).  The device job table holds per task
-// its tensor maps, sizes and output, and the item prefix offsets; items are
-// numbered task by task (tasks sorted by cost on the host, most expensive
-// first).
+// and correlate_function.c:59-83).  Here every output tile of every task is a
+// work item, computed by a cluster of two CTAs: 256 A rows and as many B rows
+// bn (a multiple of 16 up to 240) as spread the task's rows evenly over its
+// tile rows (batch_tile_rows); rank r holds A rows 128 r.. and B rows bn/2 r..
+// of the tile.  The device job table holds per task its tensor maps, sizes and
+// output, and the item prefix offsets; items are numbered task by task (tasks
+// sorted by cost on the host, most expensive first).
 //
-// Work queue: rank 0's producer thread claims the next item with an atomic
-// ticket on a global counter, decodes it into (task, A tile, B tile) and
-// writes it into the 4-slot item ring of both CTAs (the peer's copy through
-// st.shared::cluster, published by a cluster-scope release arrive).  In each
-// CTA the TMA thread, the unpack warps and the epilogue warps (and in rank 0
-// the MMA thread) pop the same items in the same order, and each releases
-// the slot on rank 0's barrier when done with its item.  A ticket past the
-// last item pushes an end marker.
+// Work queue: rank 0's queue warp runs ahead of the others, claims the next
+// item with an atomic ticket on a global counter, decodes it into (task, A row,
+// B row) and writes it into the 4-slot item ring of both CTAs (the peer's copy
+// through st.shared::cluster, published by a cluster-scope release arrive).  In
+// each CTA the TMA thread, the unpack warps and the epilogue warps (and in rank
+// 0 the MMA warp) pop the same items in the same order, and each releases the
+// slot on rank 0's barrier when done with its item.  A ticket past the last
+// item pushes an end marker.  With the TMA thread claiming and decoding its
+// items itself (an atomic and a binary search, ~4 us) and 240-row tiles
+// throughout, 300 tasks of 64-2,048 SNPs took 567 us against 533 (reference
+// mode 647 / 614).
 //
-// Roles per CTA (576 threads in R2_EXACT, 704 in R2_REFERENCE): warp 0 queue
-// (rank 0) and TMA of the CTA's rows, warp 1 TMEM and (rank 0) the MMAs,
+// Roles per CTA (608 threads in R2_EXACT, 736 in R2_REFERENCE): warp 0 TMA of
+// the CTA's rows, warp 1 TMEM and (rank 0) the MMAs,
 // warps 2-9 unpack in four groups taking the 256-sample stages in turn (each
 // thread whole rows), warps 10-17 (10-21) epilogue, two (three) per TMEM lane
-// quarter.  TMEM: two 240-column accumulators
+// quarter, the last warp (rank 0) the queue.  TMEM: two accumulators
 // (columns 0 and 256), so a tile's epilogue overlaps the next tile's MMAs,
 // and the scale factors at columns 496-511.  Every wait is bounded and no
 // thread returns early: both CTAs meet at the cluster barriers at start and
 // end on every path.
 #include "epilogue.cuh"
 #include "mxf4_rows.cuh"
+#include "mxf4_tiles.cuh"
 #include "qld_kernels.h"
 #include "tcgen05.cuh"
 
@@ -44,13 +49,13 @@ namespace {
 
 using namespace tc;
 
-constexpr int BM = 256, BN = 240;           // work item: output tile of a pair
+constexpr int BM = RowTiles::BM, BN = 240;  // work item: output tile of a pair (up to)
 constexpr int HM = 128, HN = 120;           // A and B rows held by each CTA
 constexpr int PW = 8;                       // packed words per row per packed stage
 constexpr int SUB = 2;                      // unpacked stages (256 samples) per packed stage
 constexpr int UST = 4;                      // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;       // 8 KB
-constexpr int P_TX = (HM + HN) * PW * 8;    // 15.5 KB delivered per stage
+constexpr int P_MAX = (HM + HN) * PW * 8;   // up to 15.5 KB delivered per stage
 constexpr int P_BYTES = 16384;              // stage stride: A rows, then B rows
 constexpr int UA_BYTES = HM * 128;          // 16 KB: 256 E2M1 per row
 constexpr int U_BYTES = (HM + HN) * 128;    // 31 KB: A rows, then B rows
@@ -59,18 +64,15 @@ constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS;
 constexpr int GROUP_THREADS = GROUP_WARPS * 32;
 constexpr int FIRST_UNPACK_WARP = 2;
 constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
-constexpr int NROWS = HM + HN;                                // rows per stage
-constexpr int TASKS = (NROWS + GROUP_THREADS - 1) / GROUP_THREADS;
+constexpr int TASKS = (HM + HN + GROUP_THREADS - 1) / GROUP_THREADS;   // rows per thread
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_STRIDE = 256;
 constexpr uint32_t SF_COL = 496;
-constexpr uint32_t IDESC_EVEN = idesc_mxf4_sf(BM, BN, 0);   // k-steps 0, 2: scale bytes 0-1
-constexpr uint32_t IDESC_ODD = idesc_mxf4_sf(BM, BN, 2);    // k-steps 1, 3: scale bytes 2-3
 constexpr int COLS_N = 256;                                  // epilogue column factors (BN used)
 constexpr uint16_t BOTH = 0x3;                               // CTA mask of a commit to both ranks
 constexpr int QSLOTS = 4;                                    // item ring depth
-// arrivals on rank 0's slot-free barrier per item: rank 0's MMA thread,
-// unpack and epilogue warps; rank 1's TMA thread, unpack and epilogue warps
+// arrivals on rank 0's slot-free barrier per item: rank 0's MMA warp; both
+// CTAs' TMA threads, unpack and epilogue warps
 // Epilogue warps per r^2 mode: eight in R2_EXACT, twelve in R2_REFERENCE,
 // whose longer per-pair sequence leaves items below ~6,000 samples waiting
 // on their epilogue (300-task mix, one-column arithmetic: 689 us against 706
@@ -81,8 +83,9 @@ template <int MODE>
 struct Roles {
     static constexpr int EPI_WARPS = MODE == R2_REFERENCE ? 12 : 8;
     static constexpr int EPI_THREADS = EPI_WARPS * 32;
-    static constexpr int THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;   // 576 or 704
-    static constexpr int ITEM_USERS = 2 * (1 + UNPACK_WARPS + EPI_WARPS);
+    static constexpr int QUEUE_WARP = FIRST_EPI_WARP + EPI_WARPS;
+    static constexpr int THREADS = (QUEUE_WARP + 1) * 32;               // 608 or 736
+    static constexpr int ITEM_USERS = 2 * (1 + UNPACK_WARPS + EPI_WARPS) + 1;
     static_assert(EPI_WARPS % 4 == 0 && EPI_THREADS >= COLS_N, "epilogue split");
 };
 
@@ -103,7 +106,7 @@ struct Smem {
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
     static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
-                      P_TX <= P_BYTES && OFF_ITEMS % 16 == 0,
+                      P_MAX <= P_BYTES && OFF_ITEMS % 16 == 0,
                   "swizzled stages must start on 1024-byte boundaries");
     // group g takes sub-stage g % 2 of packed stages g / 2, g / 2 + 2, ...: a
     // slot always belongs to the same two groups
@@ -112,28 +115,53 @@ struct Smem {
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
 static_assert(SUB == 2, "work split");
 
+// A work item: task (< 0: end of the queue), its tile's first A and B row, and
+// the packed stages (low 24 bits) and tile rows / 16 (high 8) of the task.
 struct Item {
-    int job, ta, tb, np;   // job < 0: end of the queue
+    int job, a_row, b_row, shape;
+    __device__ __forceinline__ int np() const { return shape & 0xFFFFFF; }
+    __device__ __forceinline__ int bn() const { return (shape >> 24) * 16; }
 };
 static_assert(sizeof(Item) == 16, "an item is one 16-byte record");
 
-// (job, ta, tb) of global item g: binary search of the item prefix, then the
-// job's own B-tile-row-first tile list.
-__device__ __forceinline__ Item decode_item(const BatchJob *jobs, int njobs, long long g) {
-    int lo = 0, hi = njobs - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (jobs[mid].item0 <= g) lo = mid;
-        else hi = mid - 1;
+// Global item g, found by the whole warp: a 32-way search of the item prefix
+// (two or three rounds of loads instead of log2(njobs)), then the job's own
+// B-tile-row-first tile list.
+__device__ __forceinline__ Item decode_item(const BatchJob *jobs, int njobs, long long g,
+                                            int lane) {
+    int lo = 0, n = njobs;                   // the job is in [lo, lo + n)
+    while (n > 1) {
+        const int step = (n + 31) / 32, at = lo + lane * step;
+        const bool below = at < lo + n && jobs[at].item0 <= g;
+        const int k = __popc(__ballot_sync(0xffffffffu, below)) - 1;   // lane 0 is always below
+        n = min(step, n - k * step);
+        lo += k * step;
     }
     const BatchJob &J = jobs[lo];
-    const TileList<BM, BN> tl{(J.m + BM - 1) / BM, 0, (J.n + BN - 1) / BN, J.symmetric, 0};
+    const RowTiles tl{J.m, 0, J.n, J.bn, J.symmetric, 0};
     Item it;
     it.job = lo;
-    tl.decode((int)(g - J.item0), it.ta, it.tb);
-    it.np = (J.K + PW - 1) / PW;
+    int t = 0, base = 0;
+    tl.decode_from((int)(g - J.item0), it.a_row, it.b_row, t, base);
+    it.shape = (J.K + PW - 1) / PW | (J.bn / 16) << 24;
     return it;
 }
+
+// What the epilogue needs of a task, in registers: read through the table, the
+// fields come from memory again after every store to the task's outputs
+// (300-task batch 533 against 504 us).
+struct JobFields {
+    const uint32_t *bcA, *bcB;
+    float *r2;
+    uint32_t *counts;
+    long long ldr, ldc;
+    int m, n, S, symmetric;
+    float threshold;
+    BatchSummary *summary;
+    __device__ __forceinline__ explicit JobFields(const BatchJob &J)
+        : bcA(J.bcA), bcB(J.bcB), r2(J.r2), counts(J.counts), ldr(J.ldr), ldc(J.ldc), m(J.m),
+          n(J.n), S(J.S), symmetric(J.symmetric), threshold(J.threshold), summary(J.summary) {}
+};
 
 template <int MODE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Roles<MODE>::THREADS, 1)
@@ -205,41 +233,53 @@ k_ld_batch(const BatchParams bp) {
     cluster_sync_all();
     tc_fence_after();
 
-    if (warp == 0) {
-        // ------------------------------- work queue (rank 0) + TMA producer --
-        if (lane == 0) {
-            int gp = 0;
+    if (warp == R::QUEUE_WARP) {
+        // ------------------------------------------- work queue (rank 0) --
+        if (rank == 0) {
             bool ok = true;
             for (int qi = 0;; ++qi) {
                 const int slot = qi % QSLOTS;
-                Item it;
-                if (rank == 0) {
-                    if (qi >= QSLOTS &&
-                        !mbar_wait_acq_cluster(smem_u32(&iempty[slot]), ((qi / QSLOTS) - 1) & 1,
-                                               limit, bp.status)) {
-                        flag_error(bp.status, ST_TIMEOUT_EMPTY);
+                if (qi >= QSLOTS) {
+                    const bool free = mbar_wait_acq_cluster(smem_u32(&iempty[slot]),
+                                                            ((qi / QSLOTS) - 1) & 1, limit,
+                                                            bp.status);
+                    if (!__all_sync(0xffffffffu, free)) {
+                        if (lane == 0) flag_error(bp.status, ST_TIMEOUT_EMPTY);
                         ok = false;
                     }
-                    const long long g =
-                        ok ? (long long)atomicAdd(bp.queue, 1ull) : (long long)bp.nitems;
-                    if (g < bp.nitems) it = decode_item(bp.jobs, bp.njobs, g);
-                    else it.job = -1, it.ta = it.tb = it.np = 0;
+                }
+                long long g = (long long)bp.nitems;
+                if (ok && lane == 0) g = (long long)atomicAdd(bp.queue, 1ull);
+                g = __shfl_sync(0xffffffffu, g, 0);
+                Item it{-1, 0, 0, 0};
+                if (g < bp.nitems) it = decode_item(bp.jobs, bp.njobs, g, lane);
+                if (lane == 0) {
                     items[slot] = it;
                     mbar_arrive(smem_u32(&ifull[slot]));   // release: the item is visible
                     st_rank_and_arrive(smem_u32(&items[slot]),
-                                       make_int4(it.job, it.ta, it.tb, it.np),
+                                       make_int4(it.job, it.a_row, it.b_row, it.shape),
                                        smem_u32(&ifull[slot]), 1);
-                } else {
-                    if (!wait_item(qi)) {
-                        flag_error(bp.status, ST_TIMEOUT_FULL);
-                        break;
-                    }
-                    it = items[slot];
                 }
+                __syncwarp();
+                if (it.job < 0) break;
+            }
+        }
+    } else if (warp == 0) {
+        // --------------------------------------------------- TMA producer --
+        if (lane == 0) {
+            int gp = 0;
+            bool ok = true;
+            for (int qi = 0; ok; ++qi) {
+                if (!wait_item(qi)) {
+                    flag_error(bp.status, ST_TIMEOUT_FULL);
+                    break;
+                }
+                const Item it = items[qi % QSLOTS];
                 if (it.job < 0) break;
                 const BatchJob &J = bp.jobs[it.job];
-                const int ra = it.ta * BM + (int)rank * HM, rb = it.tb * BN + (int)rank * HN;
-                for (int kp = 0; kp < it.np && ok; ++kp, ++gp) {
+                const int hn = it.bn() / 2, np = it.np();
+                const int ra = it.a_row + (int)rank * HM, rb = it.b_row + (int)rank * hn;
+                for (int kp = 0; kp < np; ++kp, ++gp) {
                     const int s = gp % PST;
                     if (gp >= PST && !mbar_wait(smem_u32(&pempty[s]), ((gp / PST) - 1) & 1,
                                                 limit, bp.status)) {
@@ -249,14 +289,11 @@ k_ld_batch(const BatchParams bp) {
                     }
                     const uint32_t fb = smem_u32(&pfull[s]);
                     const uint32_t dst = smem_u32(smem + L::OFF_P + s * P_BYTES);
-                    mbar_arrive_expect_tx(fb, P_TX);
+                    mbar_arrive_expect_tx(fb, PA_BYTES + (uint32_t)(hn * PW * 8));
                     tma_load_2d(dst, &J.tmA, kp * PW, ra, fb);
                     tma_load_2d(dst + PA_BYTES, &J.tmB, kp * PW, rb, fb);
                 }
-                if (rank == 1) {
-                    release_item(qi);
-                    if (!ok) break;
-                }
+                release_item(qi);
             }
             for (int g = gp > PST ? gp - PST : 0; g < gp; ++g)
                 if (!mbar_wait(smem_u32(&pfull[g % PST]), (g / PST) & 1, kDrainCycles, nullptr)) {
@@ -280,6 +317,9 @@ k_ld_batch(const BatchParams bp) {
                 }
                 const Item it = items[slot];
                 if (it.job < 0) break;
+                const uint32_t even = idesc_mxf4_sf(BM, it.bn(), 0);   // k-steps 0, 2: scale bytes 0-1
+                const uint32_t odd = idesc_mxf4_sf(BM, it.bn(), 2);    // k-steps 1, 3: scale bytes 2-3
+                const int nu = it.np() * SUB;
                 const int ab = it_n & 1;
                 if (it_n >= 2) {
                     const bool free = mbar_wait(smem_u32(&accempty[ab]), ((it_n >> 1) - 1) & 1,
@@ -291,7 +331,7 @@ k_ld_batch(const BatchParams bp) {
                 }
                 tc_fence_after();
                 const uint32_t d = tmem + (uint32_t)ab * ACC_STRIDE;
-                for (int u = 0; u < it.np * SUB; ++u) {
+                for (int u = 0; u < nu; ++u) {
                     const bool full = mbar_wait(smem_u32(&ufull[s]), ph, limit, bp.status);
                     if (!__all_sync(0xffffffffu, full)) {
                         if (lane == 0) flag_error(bp.status, ST_TIMEOUT_UNPACK);
@@ -304,7 +344,7 @@ k_ld_batch(const BatchParams bp) {
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
                             tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
-                                                (kk & 1) ? IDESC_ODD : IDESC_EVEN,
+                                                (kk & 1) ? odd : even,
                                                 (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
                         tc_commit_pair(smem_u32(&uempty[s]), BOTH);
                     }
@@ -335,7 +375,8 @@ k_ld_batch(const BatchParams bp) {
             }
             const Item it = items[qi % QSLOTS];
             if (it.job < 0) break;
-            for (int kp = 0; kp < it.np; ++kp, ++gp) {
+            const int np = it.np(), nrows = HM + it.bn() / 2;
+            for (int kp = 0; kp < np; ++kp, ++gp) {
                 if ((gp & 1) != grp / SUB) continue;
                 const int ps = gp % PST;
                 const bool got = mbar_wait(smem_u32(&pfull[ps]), (gp / PST) & 1, limit, bp.status);
@@ -354,7 +395,7 @@ k_ld_batch(const BatchParams bp) {
                     break;
                 }
                 mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(
-                    rows, NROWS, smem + L::OFF_P + ps * P_BYTES, smem + L::OFF_U + us * U_BYTES,
+                    rows, nrows, smem + L::OFF_P + ps * P_BYTES, smem + L::OFF_U + us * U_BYTES,
                     grp % SUB);
                 fence_proxy_async_smem();
                 __syncwarp();
@@ -388,12 +429,15 @@ k_ld_batch(const BatchParams bp) {
             const Item it = items[qi % QSLOTS];
             named_bar_sync(1, R::EPI_THREADS);
             if (*epi_fail || it.job < 0) break;
-            const BatchJob &J = bp.jobs[it.job];
+            const JobFields J(bp.jobs[it.job]);
             const int ab = qi & 1;
+            const int a = it.a_row + (int)rank * HM + q * 32 + lane;
+            const bool a_ok = a < J.m;
+            const uint32_t ca = a_ok ? J.bcA[a] : 0u;
             bool special = false;
             if (et < COLS_N) {   // every column factor the chunks read; 0 past the tile and the task
-                const int b = it.tb * BN + et;
-                const uint32_t cb = (et < BN && b < J.n) ? J.bcB[b] : 0u;
+                const int b = it.b_row + et;
+                const uint32_t cb = (et < it.bn() && b < J.n) ? J.bcB[b] : 0u;
                 if constexpr (MODE == R2_EXACT)
                     special = epi::store_col_f32(colsf, et, cb, J.S);
                 else
@@ -410,14 +454,11 @@ k_ld_batch(const BatchParams bp) {
             } else {
                 __syncwarp();
                 tc_fence_after();
-                const int a = it.ta * BM + (int)rank * HM + q * 32 + lane;
-                const bool a_ok = a < J.m;
-                const uint32_t ca = a_ok ? J.bcA[a] : 0u;
                 const epi::ARowR ra = epi::make_arow_ref(ca, J.S);
                 const epi::ARowF raf = epi::make_arow_f32(ca, J.S);
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                const int n_tile = it.tb * BN + BN < J.n ? it.tb * BN + BN : J.n;
+                const int n_tile = it.b_row + it.bn() < J.n ? it.b_row + it.bn() : J.n;
                 const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
                 epi::SumAcc acc;
                 // Chunks of 16 columns, in reference mode of 8 (more columns spill:
@@ -425,20 +466,20 @@ k_ld_batch(const BatchParams bp) {
                 // reference mode 668 against 647)
                 constexpr int CW = MODE == R2_EXACT ? 16 : 8;
 #pragma unroll 1
-                for (int c = colh; c < BN / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
+                for (int c = colh; c < it.bn() / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
                     uint32_t v[CW];
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special, c * CW,
-                                           it.tb * BN + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
+                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
+                                           c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
                                            J.ldr, J.counts, J.ldc, 0, J.S);
                         if (J.summary)
-                            acc.fold(v, it.tb * BN + c * CW, a, a_ok, J.n, J.symmetric,
+                            acc.fold(v, it.b_row + c * CW, a, a_ok, J.n, J.symmetric,
                                      J.threshold);
                     } else {
                         // the F32 accumulators hold the counts as floats
-                        epi::chunk_ref<0, true, CW>(v, ra, colsr, c * CW, it.tb * BN + c * CW, a,
+                        epi::chunk_ref<0, true, CW>(v, ra, colsr, c * CW, it.b_row + c * CW, a,
                                                     a_ok, n_tile, dlo, dhi, J.r2, J.ldr,
                                                     J.counts, J.ldc, 0, J.S);
                     }
@@ -508,6 +549,17 @@ cudaError_t launch_mode(const BatchParams &bp, int max_ctas, cudaStream_t st) {
 
 const KernelShape kBatchShape = {BM, BN, PW, HM, HN, 64};
 const int kBatchMaxSamples = 1 << 24;
+
+// As few tile rows as 240-row tiles need, of (nearly) equal height: 250 B rows
+// are two tiles of 128, not 240 + 10, and 64 are one of 64, so padding rows are
+// not unpacked, multiplied or run through the epilogue.
+int batch_tile_rows(int n) {
+    const int rows = (n + BN - 1) / BN;
+    return rows < 1 ? 16 : ((n + rows - 1) / rows + 15) / 16 * 16;
+}
+long long batch_tiles(int m, int n, int symmetric) {
+    return RowTiles{m, 0, n, batch_tile_rows(n), symmetric, 0}.count();
+}
 
 cudaError_t launch_batch(const BatchParams &bp, int r2_mode, int max_ctas, cudaStream_t st) {
     return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE>(bp, max_ctas, st)

@@ -619,7 +619,7 @@ int prepare_batch(qld_ctx *c, const qld_ld_args *jobs, int njobs, std::vector<Ba
             return set_err(c, QLD_ERR_UNSUPPORTED,
                            "batch job %d: the forced kernel is not exact for K*64 = %lld samples",
                            j, (long long)a.K * 64);
-        tiles[j] = (a.m == 0 || a.n == 0) ? 0 : tile_count(t, ks.bm, ks.bn, 0, a.n);
+        tiles[j] = (a.m == 0 || a.n == 0) ? 0 : batch_tiles(a.m, a.n, a.symmetric);
         if (variant != QLD_KERNEL_FP4 || (long long)a.K * 64 > kBatchMaxSamples) {
             if (tiles[j] > 0) routed.push_back({t, a.r2, a.ldr, a.counts, a.ldc});
             continue;
@@ -641,11 +641,12 @@ int prepare_batch(qld_ctx *c, const qld_ld_args *jobs, int njobs, std::vector<Ba
         J.bcA = a.bcA; J.bcB = a.bcB; J.r2 = a.r2; J.counts = a.counts;
         J.ldr = a.ldr; J.ldc = a.ldc; J.item0 = items;
         J.m = a.m; J.n = a.n; J.K = a.K; J.S = a.S; J.symmetric = a.symmetric;
+        J.bn = batch_tile_rows(a.n);
         if (tiles[j] > 0) {
             int rc;
             if ((rc = make_tmap(c, &J.tmA, a.A, a.m, a.K, a.lda, ks.box_words, ks.box_rows_a,
                                 ks.swizzle)) ||
-                (rc = make_tmap(c, &J.tmB, a.B, a.n, a.K, a.ldb, ks.box_words, ks.box_rows_b,
+                (rc = make_tmap(c, &J.tmB, a.B, a.n, a.K, a.ldb, ks.box_words, J.bn / 2,
                                 ks.swizzle)))
                 return rc;
         }

@@ -67,6 +67,7 @@ struct BatchJob {
     long long ldr, ldc;
     long long item0;
     int m, n, K, S, symmetric;
+    int bn;                    // B rows per tile (batch_tile_rows), tmB's box: bn / 2
     float threshold;           // with summary: the n_above threshold
     BatchSummary *summary;     // NULL: none
 };
@@ -80,7 +81,10 @@ struct BatchParams {
     long long timeout_cycles;
 };
 
-extern const KernelShape kBatchShape;   // 256 x 240 tiles on SM pairs, the 4-bit path
+extern const KernelShape kBatchShape;   // up to 256 x 240 tiles on SM pairs, the 4-bit path
+// B rows per tile of a batched task of n B rows, and its number of tiles.
+int batch_tile_rows(int n);
+long long batch_tiles(int m, int n, int symmetric);
 extern const int kBatchMaxSamples;      // K * 64 limit of a batched task (2^24)
 
 // Persistent batched launch over all items of bp.jobs (max_ctas > 0 caps the grid).

@@ -181,7 +181,7 @@ int launch_slot(qld_server *s, int si) {
         const Query &q = sl.qs[i];
         const int m = q.q.a1 - q.q.a0, n = q.q.b1 - q.q.b0;
         const int sym = (q.q.a0 == q.q.b0 && q.q.a1 == q.q.b1);
-        tiles[i] = tc::TileList<256, 240>{(m + 255) / 256, 0, (n + 239) / 240, sym, 0}.count();
+        tiles[i] = batch_tiles(m, n, sym);
         cost[i] = tiles[i] * (long long)tables[q.q.table].K;
         order[i] = i;
     }
@@ -198,7 +198,7 @@ int launch_slot(qld_server *s, int si) {
         memset(&J, 0, sizeof J);
         const uint64_t *A = T.d + (size_t)q.q.a0 * T.lda, *B = T.d + (size_t)q.q.b0 * T.lda;
         if (!encode_map(s, &J.tmA, A, m, T.K, T.lda, kBatchShape.box_rows_a) ||
-            !encode_map(s, &J.tmB, B, n, T.K, T.lda, kBatchShape.box_rows_b))
+            !encode_map(s, &J.tmB, B, n, T.K, T.lda, batch_tile_rows(n) / 2))
             return QLD_ERR_CUDA;
         J.bcA = T.bc + q.q.a0;
         J.bcB = T.bc + q.q.b0;
@@ -206,6 +206,7 @@ int launch_slot(qld_server *s, int si) {
         J.ldr = m;
         J.item0 = items;
         J.m = m; J.n = n; J.K = T.K; J.S = T.S; J.symmetric = sym;
+        J.bn = batch_tile_rows(n);
         J.threshold = q.q.threshold;
         J.summary = sl.dSum + i;
         items += tiles[i];
