@@ -68,7 +68,7 @@ constexpr int PW = 8;                    // packed words per row per packed stag
 constexpr int SUB = 2;                   // unpacked stages (256 samples) per packed stage
 constexpr int UST = 4;                   // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;    // 8 KB
-constexpr int P_TX = (HM + HN) * PW * 8; // 15.5 KB delivered per stage
+constexpr int P_MAX = (HM + HN) * PW * 8;   // up to 15.5 KB delivered per stage
 constexpr int P_BYTES = 15872;           // stage stride: A rows, then B rows (a multiple of 512)
 constexpr int UA_BYTES = HM * 128;       // 16 KB: 256 E2M1 per row
 constexpr int U_BYTES = (HM + HN) * 128; // 31 KB: A rows, then B rows
@@ -79,13 +79,10 @@ constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
 constexpr int EPILOGUE = EPI_WARPS * 32;
 constexpr int THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;   // 576
 constexpr int GROUP_THREADS = GROUP_WARPS * 32;              // unpackers per stage
-constexpr int NROWS = HM + HN;                               // rows per stage
-constexpr int TASKS = (NROWS + GROUP_THREADS - 1) / GROUP_THREADS;
+constexpr int TASKS = (HM + HN + GROUP_THREADS - 1) / GROUP_THREADS;   // rows per thread
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_STRIDE = 256;     // accumulator buffers at columns 0 and 256
 constexpr uint32_t SF_COL = 496;         // 16 columns of scale factors
-constexpr uint32_t IDESC_EVEN = idesc_mxf4_sf(BM, BN, 0);   // k-steps 0, 2: scale bytes 0-1
-constexpr uint32_t IDESC_ODD = idesc_mxf4_sf(BM, BN, 2);    // k-steps 1, 3: scale bytes 2-3
 constexpr int COLS_N = 256;              // epilogue column factors (BN used)
 constexpr uint16_t BOTH = 0x3;           // CTA mask of a commit to both ranks
 
@@ -106,7 +103,7 @@ struct Smem {
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
     static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
-                      P_BYTES % 512 == 0 && P_TX <= P_BYTES,
+                      P_BYTES % 512 == 0 && P_MAX <= P_BYTES,
                   "swizzled stages must start on whole swizzle atoms");
     // a group sees every (GROUPS / 2)-th packed stage or so: a slot must
     // always belong to the same groups for its phase bit to be enough
@@ -117,7 +114,8 @@ static_assert(SUB == 2 && EPILOGUE >= COLS_N && EPI_WARPS % 4 == 0, "work split"
 
 // BAND: a band's launch (its window and tiles); otherwise two regions or a
 // single region.  One kernel for both ran the other two 1.2 % slower.
-template <int MODE, bool BAND>
+// FULL: 240-row tiles, else tl.bn (a multiple of 16).
+template <int MODE, bool BAND, bool FULL>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const LdParams p, const RowTiles all, const int ntiles) {
@@ -138,6 +136,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int pair = (int)cluster_id_x(), npairs = (int)cluster_count_x();
     RowTiles tl = all;
     if (!BAND) tl.band = 0;
+    if (FULL) tl.bn = BN;
+    const int bn = tl.bn, hn = bn / 2;
     const int dlo = diag_lo(p.symmetric, tl.band), dhi = diag_hi(tl.band);
     const int my_tiles = pair < ntiles ? (ntiles - pair + npairs - 1) / npairs : 0;
 
@@ -190,7 +190,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             for (int i = 0; i < my_tiles && ok; ++i) {
                 int a_row, b_row;
                 tl.decode_from(pair + i * npairs, a_row, b_row, cur_t, cur_base);
-                const int ra = a_row + (int)rank * HM, rb = b_row + (int)rank * HN;
+                const int ra = a_row + (int)rank * HM, rb = b_row + (int)rank * hn;
                 for (int kp = 0; kp < np; ++kp, ++gp) {
                     const int s = gp % PST;
                     if (gp >= PST && !mbar_wait(smem_u32(&pempty[s]), ((gp / PST) - 1) & 1,
@@ -201,7 +201,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     }
                     const uint32_t fb = smem_u32(&pfull[s]);
                     const uint32_t dst = smem_u32(smem + L::OFF_P + s * P_BYTES);
-                    mbar_arrive_expect_tx(fb, P_TX);
+                    mbar_arrive_expect_tx(fb, PA_BYTES + (uint32_t)(hn * PW * 8));
                     tma_load_2d(dst, &tmA, kp * PW, ra, fb);
                     tma_load_2d(dst + PA_BYTES, &tmB, kp * PW, rb, fb);
                 }
@@ -217,6 +217,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         // ------------------------------------------- MMA issuer (rank 0) --
         if (rank == 0) {
             const uint32_t sf = tmem + SF_COL;
+            const uint32_t even = idesc_mxf4_sf(BM, bn, 0);   // k-steps 0, 2: scale bytes 0-1
+            const uint32_t odd = idesc_mxf4_sf(BM, bn, 2);    // k-steps 1, 3: scale bytes 2-3
             const uint32_t a_lo = sw128_desc_lo(smem_u32(smem + L::OFF_U));
             uint32_t s = 0, ph = 0;      // unpacked stage and its phase
             bool ok = true;
@@ -246,7 +248,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
 #pragma unroll
                         for (int kk = 0; kk < 4; ++kk)
                             tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
-                                                (kk & 1) ? IDESC_ODD : IDESC_EVEN,
+                                                (kk & 1) ? odd : even,
                                                 (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
                         tc_commit_pair(smem_u32(&uempty[s]), BOTH);
                     }
@@ -282,7 +284,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 if (lane == 0) flag_error(p.status, ST_TIMEOUT_MMA);
                 break;
             }
-            mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(rows, NROWS, smem + L::OFF_P + ps * P_BYTES,
+            mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(rows, HM + hn, smem + L::OFF_P + ps * P_BYTES,
                                                         smem + L::OFF_U + us * U_BYTES, gu & 1);
             fence_proxy_async_smem();
             __syncwarp();
@@ -307,7 +309,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int a = a_row + (int)rank * HM + q * 32 + lane, b = b_row + et;
             ca = a < p.m ? p.bcA[a] : 0u;
             // every column factor the chunks read; 0 past the tile and the task
-            cb = et < BN && b < p.n ? p.bcB[b] : 0u;
+            cb = et < bn && b < p.n ? p.bcB[b] : 0u;
         };
         epi::ARowR ra{};
         epi::ARowF raf{};
@@ -346,13 +348,13 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 uint8_t *base = smem + L::OFF_ROWS + ab * L::ROWS_BYTES;
                 const uint32_t tbase =
                     tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                const int n_tile = b_tile + BN < p.n ? b_tile + BN : p.n;
+                const int n_tile = b_tile + bn < p.n ? b_tile + bn : p.n;
                 // Chunks of 16 columns, in reference mode of 8: their packed
                 // arithmetic keeps more values live (16 columns spill: band of
                 // 1,000 in reference mode 244 us against 241).
                 constexpr int CW = MODE == R2_EXACT ? 16 : 8;
 #pragma unroll 1
-                for (int c = colh; c < BN / CW; c += EPI_WARPS / 4) {
+                for (int c = colh; c < bn / CW; c += EPI_WARPS / 4) {
                     uint32_t v[CW];
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
@@ -395,38 +397,40 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     }
 }
 
-int g_max_pairs = 0;
+// Clusters that run at once, asked of the driver once.
+int max_pairs() {
+    static std::atomic<int> known;
+    int n = known.load(std::memory_order_relaxed);
+    if (n > 0) return n;
+    auto kern = k_ld_mxf4_pair<R2_EXACT, false, true>;
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(2 * (sms / 2), 1, 1);
+    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.dynamicSmemBytes = Smem<R2_EXACT>::BYTES;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             Smem<R2_EXACT>::BYTES) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
+        (void)cudaGetLastError();
+        n = sms / 2;
+    }
+    known.store(n, std::memory_order_relaxed);
+    return n;
+}
 
-template <int MODE, bool BAND>
+template <int MODE, bool BAND, bool FULL>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
-                        int tiles_b, cudaStream_t st) {
-    auto kern = k_ld_mxf4_pair<MODE, BAND>;
+                        const RowTiles &tl, cudaStream_t st) {
+    auto kern = k_ld_mxf4_pair<MODE, BAND, FULL>;
     static std::atomic<unsigned long long> allowed;
     cudaError_t e = allow_smem(kern, Smem<MODE>::BYTES, allowed);
     if (e != cudaSuccess) return e;
-    if (g_max_pairs == 0) {
-        int dev = 0, sms = 0;
-        if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
-        if ((e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) !=
-            cudaSuccess)
-            return e;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * (sms / 2), 1, 1);
-        cfg.blockDim = dim3(THREADS, 1, 1);
-        cfg.dynamicSmemBytes = Smem<MODE>::BYTES;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
-            (void)cudaGetLastError();
-            n = sms / 2;
-        }
-        g_max_pairs = n;
-    }
-    const long long last = ((long long)p.tb0 + tiles_b) * BN;
-    const RowTiles tl{p.m,         p.tb0 * BN, last < p.n ? (int)last : p.n, BN,
-                      p.symmetric, p.band};
-    const int ntiles = tl.count();
+    const int ntiles = tl.count(), most = max_pairs();
     if (ntiles == 0) return cudaSuccess;
-    const int pairs = ntiles < g_max_pairs ? ntiles : g_max_pairs;
+    const int pairs = ntiles < most ? ntiles : most;
     cudaLaunchAttribute at = overlap_attr();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
@@ -438,18 +442,64 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, tl, ntiles);
 }
 
+template <int MODE>
+cudaError_t launch_tiles(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
+                         const RowTiles &tl, cudaStream_t st) {
+    if (tl.band > 0)
+        return tl.bn == BN ? launch_mode<MODE, true, true>(tmA, tmB, p, tl, st)
+                           : launch_mode<MODE, true, false>(tmA, tmB, p, tl, st);
+    return tl.bn == BN ? launch_mode<MODE, false, true>(tmA, tmB, p, tl, st)
+                       : launch_mode<MODE, false, false>(tmA, tmB, p, tl, st);
+}
+
 }  // namespace
 
 const KernelShape kMxf4PairShape = {BM, BN, PW, HM, HN, 64};
 
+// B rows per tile of a launch.  240 rows make the most of the MMAs, but a
+// launch of few tiles ends on a wave that few SM pairs work in: 90 tiles on 74
+// pairs take as long as 148.  Lower tiles fill that wave at a little more work
+// per entry, so up to sixteen waves the height with the least estimated time
+// is taken, if it saves 5 %.  The estimate (us, fitted to a sweep of 60
+// launches of 2,700 to 9,001 SNPs and K = 16, 80, 260 on a B200): waves times
+// the longer of a tile's MMAs (0.31 per 256-sample stage at 240 rows, 0.20 +
+// 0.00053 bn at fewer, 0.21 + 0.00034 bn up to 128, whose unpack takes a row
+// less per thread) and its epilogue (1.1 + 0.02 bn, reference mode 0.0405),
+// plus what the shorter adds beside it.  3,000 SNPs: K = 80 24.5 -> 20.9 us,
+// reference mode 33.2 -> 24.9; 5,286: 43.4 -> 39.5, 60.8 -> 53.8; 6,001: 52.7
+// -> 50.1, 72.6 -> 68.9; 7.5 % on average over the sweep.
+int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
+    RowTiles t = tl;
+    t.bn = BN;
+    const int most = max_pairs();
+    if (t.rows() > 64 || t.count() > 16 * most) return BN;
+    const double stages = (double)((K + PW - 1) / PW * SUB);
+    auto estimate = [&](int bn) {
+        t.bn = bn;
+        const int waves = (t.count() + most - 1) / most;
+        const double mma = stages * (bn == BN    ? 0.31
+                                     : bn > 128 ? 0.20 + 0.00053 * bn
+                                                : 0.21 + 0.00034 * bn);
+        const double epi = 1.1 + (r2_mode == R2_REFERENCE ? 0.0405 : 0.02) * bn;
+        const double a = mma > epi ? mma : epi, b = mma > epi ? epi : mma;
+        return waves * (a + 0.42 * b * b / a);
+    };
+    double best = 0.95 * estimate(BN);
+    int bn = BN;
+    for (int x = BN - 16; x >= 80; x -= 16) {
+        const double us = estimate(x);
+        if (us < best) {
+            best = us;
+            bn = x;
+        }
+    }
+    return bn;
+}
+
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
-                             int tiles_b, int r2_mode, cudaStream_t st) {
-    if (tiles_b <= 0 || p.m <= 0) return cudaSuccess;
-    if (p.band > 0)
-        return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE, true>(tmA, tmB, p, tiles_b, st)
-                                       : launch_mode<R2_EXACT, true>(tmA, tmB, p, tiles_b, st);
-    return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE, false>(tmA, tmB, p, tiles_b, st)
-                                   : launch_mode<R2_EXACT, false>(tmA, tmB, p, tiles_b, st);
+                             const RowTiles &tl, int r2_mode, cudaStream_t st) {
+    return r2_mode == R2_REFERENCE ? launch_tiles<R2_REFERENCE>(tmA, tmB, p, tl, st)
+                                   : launch_tiles<R2_EXACT>(tmA, tmB, p, tl, st);
 }
 
 }  // namespace qld

@@ -316,16 +316,19 @@ int launch_counts(qld_ctx *c, const Task &t, int b0, int b1, float *r2, long lon
                        "4-bit tensor-core kernel needs K*64 <= %d samples (K=%d)",
                        kMxf4MaxSamples, t.K);
     const KernelShape &ks = shape_of(c, variant, t, b0, b1);
-    // a launch whose tiles all run at once: smaller tiles, words split over pairs
+    // SM pairs: the launch's own tiles; all at once, smaller ones with their
+    // words split over pairs
+    const bool pair = &ks == &kMxf4PairShape;
+    RowTiles tl{t.m, b0, b1, ks.bn, t.symmetric, t.band};
     SplitPlan sp{};
-    const bool split = &ks == &kMxf4PairShape && c->sm_pair == 0 &&
-                       plan_split(RowTiles{t.m, b0, b1, 0, t.symmetric, t.band}, t.K, c->r2_mode,
-                                  &sp);
+    const bool split = pair && c->sm_pair == 0 && plan_split(tl, t.K, c->r2_mode, &sp);
+    if (split) tl.bn = sp.bn;
+    else if (pair && c->sm_pair == 0) tl.bn = pair_tile_rows(tl, t.K, c->r2_mode);
     CUtensorMap tmA, tmB;
     int rc;
     if ((rc = make_tmap(c, &tmA, t.A, t.m, t.K, t.lda, ks.box_words, ks.box_rows_a, ks.swizzle)) ||
         (rc = make_tmap(c, &tmB, t.B, t.n, t.K, t.ldb, ks.box_words,
-                        split ? sp.bn / 2 : ks.box_rows_b, ks.swizzle)))
+                        pair ? tl.bn / 2 : ks.box_rows_b, ks.swizzle)))
         return rc;
     const int tb0 = b0 / ks.bn;
     const int tiles_b = (b1 - b0 + ks.bn - 1) / ks.bn;
@@ -345,13 +348,12 @@ int launch_counts(qld_ctx *c, const Task &t, int b0, int b1, float *r2, long lon
     }
     p.status = c->d_status;
     p.timeout_cycles = c->timeout_cycles;
-    if (split) {
+    if (pair) {
         p.n = b1;                        // its tile rows need not end at b1
         cudaEvent_t e1 = nullptr;
         if ((rc = prof_begin(c, st, &e1))) return rc;
-        const cudaError_t e =
-            launch_mxf4_split(tmA, tmB, p, RowTiles{t.m, b0, b1, sp.bn, t.symmetric, t.band},
-                              sp.ks, c->r2_mode, st);
+        const cudaError_t e = split ? launch_mxf4_split(tmA, tmB, p, tl, sp.ks, c->r2_mode, st)
+                                    : launch_mxf4_pair(tmA, tmB, p, tl, c->r2_mode, st);
         if (e != cudaSuccess)
             return set_err(c, QLD_ERR_CUDA, "counts kernel launch failed: %s", cudaGetErrorString(e));
         if (e1) CUDA_TRY(c, cudaEventRecord(e1, st));
@@ -366,8 +368,7 @@ int launch_counts(qld_ctx *c, const Task &t, int b0, int b1, float *r2, long lon
         cudaEvent_t e1 = nullptr;
         if (int rc = prof_begin(c, st, &e1)) return rc;
         cudaError_t e =
-            &ks == &kMxf4PairShape    ? launch_mxf4_pair(tmA, tmB, p, nb, c->r2_mode, st)
-            : variant == QLD_KERNEL_FP4 ? launch_mxf4(tmA, tmB, p, nb, c->r2_mode, st)
+            variant == QLD_KERNEL_FP4 ? launch_mxf4(tmA, tmB, p, nb, c->r2_mode, st)
             : variant != QLD_KERNEL_MMA ? launch_popc(tmA, tmB, p, nb, c->r2_mode, st)
             : &ks == &kMmaWideShape     ? launch_mma_wide(tmA, tmB, p, nb, c->r2_mode, st)
                                         : launch_mma(tmA, tmB, p, nb, c->r2_mode, st);

@@ -45,8 +45,11 @@ cudaError_t launch_mxf4(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
 // The same tiles computed by clusters of two CTAs (one per SM, 128 A rows and
 // 120 B rows each), with the epilogue overlapping the next tile's MMAs.
 extern const KernelShape kMxf4PairShape;
+// tl: the launch's tiles (tl.bn a multiple of 16 up to 240; pair_tile_rows picks
+// it for the others of tl).
+int pair_tile_rows(const RowTiles &tl, int K, int r2_mode);
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
-                             int tiles_b, int r2_mode, cudaStream_t st);
+                             const RowTiles &tl, int r2_mode, cudaStream_t st);
 
 // The same arithmetic for a launch whose tiles all run at once: 256 x bn
 // tiles, each on a cluster of ks SM pairs that split its words.  plan_split
