@@ -123,9 +123,12 @@ __device__ __forceinline__ float4 ref_factors(uint32_t c, int S) {
     return make_float4(v, hi, __double2float_rn(__dsub_rn(i, (double)hi)), __frcp_rn(v));
 }
 
+// Returns whether the column has a NaN factor (v >= 1).
 template <class C>
-__device__ __forceinline__ void store_col_ref(const C &f, int bl, uint32_t c, int S) {
-    f.put(bl, ref_factors(c, S));
+__device__ __forceinline__ bool store_col_ref(const C &f, int bl, uint32_t c, int S) {
+    const float4 k = ref_factors(c, S);
+    f.put(bl, k);
+    return k.y != k.y;
 }
 
 // Per-thread A-row factors of the reference mode.
@@ -480,6 +483,54 @@ __device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, co
     }
 }
 
+// chunk_ref for a warp whose row and columns have no NaN factor (no fixed SNP),
+// without the counts: every pair on the fast path, in pairs of columns.  If
+// one is flagged or meets the > 1.0001 rule, the chunk's counts are loaded
+// again (reload(v)) and it goes through chunk_ref.  At S >= R2_PLAIN_S that is
+// one chunk in some hundreds; smaller S meet rounding midpoints more often.
+constexpr int R2_PLAIN_S = 256;
+template <int CW, class Reload>
+__device__ __forceinline__ void chunk_ref_plain(uint32_t (&v)[CW], const ARowR &ra,
+                                                const ColsR2 &f, int bl0, int b0, int a, bool a_ok,
+                                                int n, int dlo, int dhi, float *r2, float *o,
+                                                long long ldr, int row0, int S, Reload reload) {
+    const ARowR2 A(ra);
+    float rmax = 0.0f;
+    bool bad = false;
+#pragma unroll
+    for (int t = 0; t < CW; t += 2) {
+        f2 bx, by, bz, bw;
+        f.pair(bl0 + t, bx, by, bz, bw);
+        float q0, q1;
+        bool rd0, rd1;
+        r2_reference_ff2(pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1])), A, bx, by, bz,
+                         bw, q0, q1, rd0, rd1);
+        rmax = max3(rmax, q0, q1);
+        bad = bad || rd0 || rd1;
+        v[t] = __float_as_uint(q0);
+        v[t + 1] = __float_as_uint(q1);
+    }
+    bad = bad || rmax > __uint_as_float(0x3F800000u + 838u);
+    if (__any_sync(0xffffffffu, a_ok && bad)) {
+        reload(v);
+        chunk_ref<0, true, CW>(v, ra, f, bl0, b0, a, a_ok, n, dlo, dhi, r2, ldr, nullptr, 0, row0,
+                               S);
+        return;
+    }
+    if (!a_ok) return;
+    const bool interior = (b0 + CW - 1 < n) && (a - (b0 + CW - 1) >= dlo) && (a - b0 <= dhi);
+    if (interior) {
+#pragma unroll
+        for (int t = 0; t < CW; ++t) o[(long long)t * ldr] = __uint_as_float(v[t]);
+    } else {
+#pragma unroll
+        for (int t = 0; t < CW; ++t) {
+            const int b = b0 + t;
+            if (b < n && a - b >= dlo && a - b <= dhi) o[(long long)t * ldr] = __uint_as_float(v[t]);
+        }
+    }
+}
+
 // One 32-column chunk: accumulators v[t] (holding count << shift) of A row a
 // against B rows b0 + t (local columns bl0 + t).  Output element (b, a) goes
 // to r2[(b - row0) * ldr + a] (and counts likewise).  Only entries inside the
@@ -646,6 +697,44 @@ __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, con
     }
     if (!a_ok) return;
     float *o = r2 + (long long)(b0 - row0) * ldr + a;
+    const bool interior = (b0 + CW - 1 < n) && (a - (b0 + CW - 1) >= dlo) && (a - b0 <= dhi);
+    if (interior) {
+#pragma unroll
+        for (int t = 0; t < CW; ++t) o[(long long)t * ldr] = __uint_as_float(v[t]);
+    } else {
+#pragma unroll
+        for (int t = 0; t < CW; ++t) {
+            const int b = b0 + t;
+            if (b < n && a - b >= dlo && a - b <= dhi) o[(long long)t * ldr] = __uint_as_float(v[t]);
+        }
+    }
+}
+
+// chunk_f32 for a warp whose row and columns are not `special`, without the
+// counts and without its votes: the values as FP32 gives them, their maximum
+// folded into rmax.  A caller that finds rmax above R2_RECHECK in any lane
+// runs the tile's chunks again through chunk_f32, which overwrites them.
+constexpr float R2_RECHECK = 1.00009f;
+template <int CW>
+__device__ __forceinline__ void chunk_f32_plain(uint32_t (&v)[CW], const ARowF &ra, const ColsF &f,
+                                                int bl0, int b0, int a, bool a_ok, int n, int dlo,
+                                                int dhi, float *o, long long ldr, float S_f,
+                                                float &rmax) {
+    const f2 S2 = splat2(S_f), ca = splat2(ra.c), nca = splat2(-ra.c), ia = splat2(ra.inv);
+#pragma unroll
+    for (int t = 0; t < CW; t += 2) {
+        const ulonglong2 col = f.pair(bl0 + t);
+        const f2 cnt = pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1]));
+        const f2 nhi = mul2(nca, col.x);                       // -hi
+        const f2 lo = fma2(ca, col.x, nhi);
+        const f2 D = sub2(fma2(S2, cnt, nhi), lo);
+        float r0, r1;
+        unpack2(mul2(mul2(D, D), mul2(ia, col.y)), r0, r1);
+        rmax = max3(rmax, r0, r1);
+        v[t] = __float_as_uint(r0);
+        v[t + 1] = __float_as_uint(r1);
+    }
+    if (!a_ok) return;
     const bool interior = (b0 + CW - 1 < n) && (a - (b0 + CW - 1) >= dlo) && (a - b0 <= dhi);
     if (interior) {
 #pragma unroll

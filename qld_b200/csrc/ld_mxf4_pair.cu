@@ -115,7 +115,13 @@ static_assert(SUB == 2 && EPILOGUE >= COLS_N && EPI_WARPS % 4 == 0, "work split"
 // BAND: a band's launch (its window and tiles); otherwise two regions or a
 // single region.  One kernel for both ran the other two 1.2 % slower.
 // FULL: 240-row tiles, else tl.bn (a multiple of 16).
-template <int MODE, bool BAND, bool FULL>
+// PLAIN: a launch without counts (p.counts null; in reference mode R2_PLAIN_S <=
+// S <= 2^24) whose tiles without special rows or columns take the epilogue
+// without the rare cases' votes, flags and per-chunk addresses: 4,001 SNPs x
+// 1,920 samples 22.0 -> 18.0 us, 12,000 x 5,120 155 -> 141, band of 1,000 over
+// 50,000 x 10,001 199 -> 192, in reference mode 241 -> 222.  A branch in one
+// kernel cost the launches with counts 1 %.
+template <int MODE, bool BAND, bool FULL, bool PLAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const LdParams p, const RowTiles all, const int ntiles) {
@@ -321,7 +327,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 special = et < COLS_N && epi::store_col_f32(epi::ColsF(base, COLS_N), et, cb, p.S);
             } else {
                 ra = epi::make_arow_ref(ca, p.S);
-                if (et < COLS_N) epi::store_col_ref(epi::ColsR2(base, COLS_N), et, cb, p.S);
+                special = et < COLS_N &&
+                          epi::store_col_ref(epi::ColsR2(base, COLS_N), et, cb, p.S);
             }
         };
         if (my_tiles > 0) {
@@ -353,8 +360,34 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 // arithmetic keeps more values live (16 columns spill: band of
                 // 1,000 in reference mode 244 us against 241).
                 constexpr int CW = MODE == R2_EXACT ? 16 : 8;
+                bool full = true;                // chunks with the rare cases' bookkeeping
+                if constexpr (PLAIN) {
+                    full = cols_special ||
+                           __any_sync(0xffffffffu, MODE == R2_EXACT ? raf.special : ra.k.y != ra.k.y);
+                    const long long step = (long long)(CW * EPI_WARPS / 4) * p.ldr;
+                    float *o = p.r2 + (long long)(b_tile + colh * CW - p.out_row0) * p.ldr + a;
+                    float rmax = 0.0f;
 #pragma unroll 1
-                for (int c = colh; c < bn / CW; c += EPI_WARPS / 4) {
+                    for (int c = colh; !full && c < bn / CW; c += EPI_WARPS / 4, o += step) {
+                        const uint32_t taddr = tbase + (uint32_t)(c * CW);
+                        uint32_t v[CW];
+                        __syncwarp();
+                        tc_ld_32x32b<CW>(taddr, v);
+                        if constexpr (MODE == R2_EXACT)
+                            epi::chunk_f32_plain<CW>(v, raf, epi::ColsF(base, COLS_N), c * CW,
+                                                     b_tile + c * CW, a, a_ok, n_tile, dlo, dhi, o,
+                                                     p.ldr, (float)p.S, rmax);
+                        else
+                            epi::chunk_ref_plain<CW>(
+                                v, ra, epi::ColsR2(base, COLS_N), c * CW, b_tile + c * CW, a, a_ok,
+                                n_tile, dlo, dhi, p.r2, o, p.ldr, p.out_row0, p.S,
+                                [&](uint32_t (&w)[CW]) { tc_ld_32x32b<CW>(taddr, w); });
+                    }
+                    if (MODE == R2_EXACT && __any_sync(0xffffffffu, rmax > epi::R2_RECHECK))
+                        full = true;
+                }
+#pragma unroll 1
+                for (int c = colh; full && c < bn / CW; c += EPI_WARPS / 4) {
                     uint32_t v[CW];
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
@@ -402,7 +435,7 @@ int max_pairs() {
     static std::atomic<int> known;
     int n = known.load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = k_ld_mxf4_pair<R2_EXACT, false, true>;
+    auto kern = k_ld_mxf4_pair<R2_EXACT, false, true, true>;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
@@ -421,10 +454,10 @@ int max_pairs() {
     return n;
 }
 
-template <int MODE, bool BAND, bool FULL>
+template <int MODE, bool BAND, bool FULL, bool PLAIN>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                         const RowTiles &tl, cudaStream_t st) {
-    auto kern = k_ld_mxf4_pair<MODE, BAND, FULL>;
+    auto kern = k_ld_mxf4_pair<MODE, BAND, FULL, PLAIN>;
     static std::atomic<unsigned long long> allowed;
     cudaError_t e = allow_smem(kern, Smem<MODE>::BYTES, allowed);
     if (e != cudaSuccess) return e;
@@ -442,14 +475,14 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, tl, ntiles);
 }
 
-template <int MODE>
+template <int MODE, bool PLAIN>
 cudaError_t launch_tiles(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                          const RowTiles &tl, cudaStream_t st) {
     if (tl.band > 0)
-        return tl.bn == BN ? launch_mode<MODE, true, true>(tmA, tmB, p, tl, st)
-                           : launch_mode<MODE, true, false>(tmA, tmB, p, tl, st);
-    return tl.bn == BN ? launch_mode<MODE, false, true>(tmA, tmB, p, tl, st)
-                       : launch_mode<MODE, false, false>(tmA, tmB, p, tl, st);
+        return tl.bn == BN ? launch_mode<MODE, true, true, PLAIN>(tmA, tmB, p, tl, st)
+                           : launch_mode<MODE, true, false, PLAIN>(tmA, tmB, p, tl, st);
+    return tl.bn == BN ? launch_mode<MODE, false, true, PLAIN>(tmA, tmB, p, tl, st)
+                       : launch_mode<MODE, false, false, PLAIN>(tmA, tmB, p, tl, st);
 }
 
 }  // namespace
@@ -498,8 +531,12 @@ int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
 
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              const RowTiles &tl, int r2_mode, cudaStream_t st) {
-    return r2_mode == R2_REFERENCE ? launch_tiles<R2_REFERENCE>(tmA, tmB, p, tl, st)
-                                   : launch_tiles<R2_EXACT>(tmA, tmB, p, tl, st);
+    if (r2_mode == R2_REFERENCE)
+        return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
+                   ? launch_tiles<R2_REFERENCE, true>(tmA, tmB, p, tl, st)
+                   : launch_tiles<R2_REFERENCE, false>(tmA, tmB, p, tl, st);
+    return !p.counts ? launch_tiles<R2_EXACT, true>(tmA, tmB, p, tl, st)
+                     : launch_tiles<R2_EXACT, false>(tmA, tmB, p, tl, st);
 }
 
 }  // namespace qld
