@@ -163,7 +163,9 @@ struct JobFields {
           n(J.n), S(J.S), symmetric(J.symmetric), threshold(J.threshold), summary(J.summary) {}
 };
 
-template <int MODE>
+// PLAIN: no task has counts or a summary (in reference mode: every S within
+// R2_PLAIN_S..2^24), as ld_mxf4_pair.cu's.
+template <int MODE, bool PLAIN>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Roles<MODE>::THREADS, 1)
 k_ld_batch(const BatchParams bp) {
     using L = Smem<MODE>;
@@ -441,7 +443,7 @@ k_ld_batch(const BatchParams bp) {
                 if constexpr (MODE == R2_EXACT)
                     special = epi::store_col_f32(colsf, et, cb, J.S);
                 else
-                    epi::store_col_ref(colsr, et, cb, J.S);
+                    special = epi::store_col_ref(colsr, et, cb, J.S);
             }
             const bool cols_special = named_bar_or(1, R::EPI_THREADS, special);
             bool ready = mbar_wait(smem_u32(&accfull[ab]), (qi >> 1) & 1, limit, bp.status);
@@ -465,8 +467,34 @@ k_ld_batch(const BatchParams bp) {
                 // 32 in exact mode 620 us against 566 on 300 tasks, 16 in
                 // reference mode 668 against 647)
                 constexpr int CW = MODE == R2_EXACT ? 16 : 8;
+                bool full = true;                // chunks with the rare cases' bookkeeping
+                if constexpr (PLAIN) {
+                    full = cols_special ||
+                           __any_sync(0xffffffffu, MODE == R2_EXACT ? raf.special : ra.k.y != ra.k.y);
+                    const long long step = (long long)(CW * R::EPI_WARPS / 4) * J.ldr;
+                    float *o = J.r2 + (long long)(it.b_row + colh * CW) * J.ldr + a;
+                    float rmax = 0.0f;
 #pragma unroll 1
-                for (int c = colh; c < it.bn() / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
+                    for (int c = colh; !full && c < it.bn() / CW; c += R::EPI_WARPS / 4, o += step) {
+                        const uint32_t taddr = tbase + (uint32_t)(c * CW);
+                        uint32_t v[CW];
+                        __syncwarp();
+                        tc_ld_32x32b<CW>(taddr, v);
+                        if constexpr (MODE == R2_EXACT)
+                            epi::chunk_f32_plain<CW>(v, raf, colsf, c * CW, it.b_row + c * CW, a,
+                                                     a_ok, n_tile, dlo, dhi, o, J.ldr, (float)J.S,
+                                                     rmax);
+                        else
+                            epi::chunk_ref_plain<CW>(
+                                v, ra, colsr, c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi,
+                                J.r2, o, J.ldr, 0, J.S,
+                                [&](uint32_t (&w)[CW]) { tc_ld_32x32b<CW>(taddr, w); });
+                    }
+                    if (MODE == R2_EXACT && __any_sync(0xffffffffu, rmax > epi::R2_RECHECK))
+                        full = true;
+                }
+#pragma unroll 1
+                for (int c = colh; full && c < it.bn() / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
                     uint32_t v[CW];
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
@@ -515,9 +543,9 @@ k_ld_batch(const BatchParams bp) {
 
 int g_max_pairs = 0;
 
-template <int MODE>
+template <int MODE, bool PLAIN>
 cudaError_t launch_mode(const BatchParams &bp, int max_ctas, cudaStream_t st) {
-    auto kern = k_ld_batch<MODE>;
+    auto kern = k_ld_batch<MODE, PLAIN>;
     cudaError_t e =
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<MODE>::BYTES);
     if (e != cudaSuccess) return e;
@@ -550,6 +578,11 @@ cudaError_t launch_mode(const BatchParams &bp, int max_ctas, cudaStream_t st) {
 const KernelShape kBatchShape = {BM, BN, PW, HM, HN, 64};
 const int kBatchMaxSamples = 1 << 24;
 
+bool batch_job_plain(const BatchJob &j, int r2_mode) {
+    return !j.counts && !j.summary &&
+           (r2_mode != R2_REFERENCE || (j.S >= epi::R2_PLAIN_S && j.S <= (1 << 24)));
+}
+
 // As few tile rows as 240-row tiles need, of (nearly) equal height: 250 B rows
 // are two tiles of 128, not 240 + 10, and 64 are one of 64, so padding rows are
 // not unpacked, multiplied or run through the epilogue.
@@ -562,8 +595,11 @@ long long batch_tiles(int m, int n, int symmetric) {
 }
 
 cudaError_t launch_batch(const BatchParams &bp, int r2_mode, int max_ctas, cudaStream_t st) {
-    return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE>(bp, max_ctas, st)
-                                   : launch_mode<R2_EXACT>(bp, max_ctas, st);
+    if (r2_mode == R2_REFERENCE)
+        return bp.plain ? launch_mode<R2_REFERENCE, true>(bp, max_ctas, st)
+                        : launch_mode<R2_REFERENCE, false>(bp, max_ctas, st);
+    return bp.plain ? launch_mode<R2_EXACT, true>(bp, max_ctas, st)
+                    : launch_mode<R2_EXACT, false>(bp, max_ctas, st);
 }
 
 }  // namespace qld

@@ -96,7 +96,8 @@ __device__ __forceinline__ void st_cluster(uint32_t addr, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
 }
 
-template <int MODE>
+// PLAIN: as ld_mxf4_pair.cu's.
+template <int MODE, bool PLAIN>
 __global__ void __launch_bounds__(THREADS, 1)
 k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                 const LdParams p, const RowTiles tl, const int ks, const int pst) {
@@ -231,7 +232,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
             const int b = b_row + wt;
             const uint32_t cb = b < p.n ? p.bcB[b] : 0u;
             if constexpr (MODE == R2_EXACT) special = epi::store_col_f32(colsf, wt, cb, p.S);
-            else epi::store_col_ref(colsr, wt, cb, p.S);
+            else special = epi::store_col_ref(colsr, wt, cb, p.S);
         }
         const uint32_t ca = a_ok ? p.bcA[a] : 0u;
         if constexpr (MODE == R2_EXACT) raf = epi::make_arow_f32(ca, p.S);
@@ -301,6 +302,8 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
         const int dlo = diag_lo(p.symmetric, p.band), dhi = diag_hi(p.band);
         const int n_tile = b_row + bn < p.n ? b_row + bn : p.n;
         const int per = (chunks + ks - 1) / ks;
+        const bool full = !PLAIN || cols_special ||
+                          __any_sync(0xffffffffu, MODE == R2_EXACT ? raf.special : ra.k.y != ra.k.y);
 #pragma unroll 1
         for (int i = cg; i * ks + split < chunks; i += 4) {
             const int c = i * ks + split;
@@ -321,8 +324,26 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                         for (int t = 0; t < CW; ++t)
                             v[t] = __float_as_uint(__uint_as_float(v[t]) + part[t * HM]);
                     }
-                    // chunk_f32 re-reads the rare count it evaluates again
-                    if constexpr (MODE == R2_EXACT) tc_st_32x32b_x16(taddr, v);
+                    // the rare pairs evaluated again are read again
+                    tc_st_32x32b<CW>(taddr, v);
+                }
+                if constexpr (PLAIN) {
+                    if (!full) {
+                        float *o = p.r2 + (long long)(b_row + col - p.out_row0) * p.ldr + a;
+                        if constexpr (MODE == R2_EXACT) {
+                            float rmax = 0.0f;
+                            epi::chunk_f32_plain<CW>(v, raf, colsf, col, b_row + col, a, a_ok,
+                                                     n_tile, dlo, dhi, o, p.ldr, (float)p.S, rmax);
+                            if (!__any_sync(0xffffffffu, rmax > epi::R2_RECHECK)) continue;
+                            tc_ld_32x32b<CW>(taddr, v);
+                        } else {
+                            epi::chunk_ref_plain<CW>(
+                                v, ra, colsr, col, b_row + col, a, a_ok, n_tile, dlo, dhi, p.r2, o,
+                                p.ldr, p.out_row0, p.S,
+                                [&](uint32_t (&w)[CW]) { tc_ld_32x32b<CW>(taddr, w); });
+                            continue;
+                        }
+                    }
                 }
                 if constexpr (MODE == R2_EXACT)
                     epi::chunk_f32<CW>(v, taddr, raf, colsf, cols_special, col, b_row + col, a,
@@ -374,13 +395,12 @@ int packed_stages(int bn, int ks) {
 }
 
 // Clusters of 2 ks CTAs that run at once, asked of the driver once per ks.
-template <int MODE>
 int max_clusters(int ks) {
     static std::atomic<int> known[3];
     std::atomic<int> &slot = known[ks >> 1];
     int n = slot.load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = k_ld_mxf4_split<MODE>;
+    auto kern = k_ld_mxf4_split<R2_EXACT, true>;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_SMEM) !=
         cudaSuccess) {
         (void)cudaGetLastError();
@@ -405,10 +425,10 @@ int max_clusters(int ks) {
     return n;
 }
 
-template <int MODE>
+template <int MODE, bool PLAIN>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                         const RowTiles &tl, int ks, cudaStream_t st) {
-    auto kern = k_ld_mxf4_split<MODE>;
+    auto kern = k_ld_mxf4_split<MODE, PLAIN>;
     const int tiles = tl.count(), pst = packed_stages(tl.bn, ks);
     if (tiles == 0) return cudaSuccess;
     if (pst < 2) return cudaErrorInvalidConfiguration;
@@ -444,8 +464,8 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
 // plus 0.008 per column delivered to another pair; 0.01 per CTA.
 bool plan_split(const RowTiles &tl, int K, int r2_mode, SplitPlan *plan) {
     const int np = (K + PW - 1) / PW, nu = (K + PW / SUB - 1) / (PW / SUB);
-    const int most[3] = {max_clusters<R2_EXACT>(1), max_clusters<R2_EXACT>(2),
-                         max_clusters<R2_EXACT>(4)};
+    const int most[3] = {max_clusters(1), max_clusters(2),
+                         max_clusters(4)};
     const double per_col = r2_mode == R2_REFERENCE ? 0.034 : 0.019;
     double best = 0.0;
     bool found = false;
@@ -475,8 +495,12 @@ bool plan_split(const RowTiles &tl, int K, int r2_mode, SplitPlan *plan) {
 
 cudaError_t launch_mxf4_split(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                               const RowTiles &tl, int ks, int r2_mode, cudaStream_t st) {
-    return r2_mode == R2_REFERENCE ? launch_mode<R2_REFERENCE>(tmA, tmB, p, tl, ks, st)
-                                   : launch_mode<R2_EXACT>(tmA, tmB, p, tl, ks, st);
+    if (r2_mode == R2_REFERENCE)
+        return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
+                   ? launch_mode<R2_REFERENCE, true>(tmA, tmB, p, tl, ks, st)
+                   : launch_mode<R2_REFERENCE, false>(tmA, tmB, p, tl, ks, st);
+    return !p.counts ? launch_mode<R2_EXACT, true>(tmA, tmB, p, tl, ks, st)
+                     : launch_mode<R2_EXACT, false>(tmA, tmB, p, tl, ks, st);
 }
 
 }  // namespace qld

@@ -657,17 +657,19 @@ int prepare_batch(qld_ctx *c, const qld_ld_args *jobs, int njobs, std::vector<Ba
 }
 
 // The launch sequence of a batched call on `st`: ticket reset and the
-// persistent launch over the nb jobs at d_jobs (when they have items), then
+// persistent launch over the jobs hj (on the device: d_jobs) (when they have items), then
 // the routed tasks' own launches.
-int enqueue_batch(qld_ctx *c, const BatchJob *d_jobs, int nb, long long items,
-                  unsigned long long *d_queue, const std::vector<RoutedTask> &routed,
-                  cudaStream_t st) {
+int enqueue_batch(qld_ctx *c, const std::vector<BatchJob> &hj, const BatchJob *d_jobs,
+                  long long items, unsigned long long *d_queue,
+                  const std::vector<RoutedTask> &routed, cudaStream_t st) {
     int rc;
     if (items > 0) {
         CUDA_TRY(c, cudaMemsetAsync(d_queue, 0, sizeof(unsigned long long), st));
         BatchParams bp{};
         bp.jobs = d_jobs;
-        bp.njobs = nb;
+        bp.njobs = (int)hj.size();
+        bp.plain = 1;
+        for (const BatchJob &j : hj) bp.plain &= batch_job_plain(j, c->r2_mode);
         bp.nitems = items;
         bp.queue = d_queue;
         bp.status = c->d_status;
@@ -722,7 +724,7 @@ int build_plan(qld_ctx *c, qld_batch_plan *p, const std::vector<BatchJob> &hj, l
     cudaError_t e = cudaStreamBeginCapture(cs, cudaStreamCaptureModeRelaxed);
     if (e == cudaSuccess) {
         c->capturing = true;
-        rc = enqueue_batch(c, p->d_jobs, (int)hj.size(), items, p->d_queue, routed, cs);
+        rc = enqueue_batch(c, hj, p->d_jobs, items, p->d_queue, routed, cs);
         c->capturing = false;
         cudaGraph_t g = nullptr;
         e = cudaStreamEndCapture(cs, &g);   // ends the capture on every path
@@ -1425,7 +1427,7 @@ int qld_cuda_ld_batch(qld_ctx *c, const qld_ld_args *jobs, int njobs, void *stre
         CUDA_TRY(c, cudaMemcpyAsync(c->dJobs.p, c->hJobs.data(), sizeof(BatchJob) * (size_t)nb,
                                     cudaMemcpyHostToDevice, st));
     }
-    return enqueue_batch(c, static_cast<const BatchJob *>(c->dJobs.p), nb, items,
+    return enqueue_batch(c, c->hJobs, static_cast<const BatchJob *>(c->dJobs.p), items,
                          static_cast<unsigned long long *>(c->dQueue.p), routed, st);
 }
 

@@ -79,6 +79,7 @@ struct BatchParams {
     const BatchJob *jobs;
     int njobs;
     long long nitems;
+    int plain;                   // every job is batch_job_plain
     unsigned long long *queue;   // work-queue ticket counter, zero at launch
     unsigned *status;
     long long timeout_cycles;
@@ -87,6 +88,9 @@ struct BatchParams {
 extern const KernelShape kBatchShape;   // up to 256 x 240 tiles on SM pairs, the 4-bit path
 // B rows per tile of a batched task of n B rows, and its number of tiles.
 int batch_tile_rows(int n);
+// Whether a job needs neither counts nor a summary, nor (in reference mode) an S
+// the plain epilogue does not take.
+bool batch_job_plain(const BatchJob &j, int r2_mode);
 long long batch_tiles(int m, int n, int symmetric);
 extern const int kBatchMaxSamples;      // K * 64 limit of a batched task (2^24)
 

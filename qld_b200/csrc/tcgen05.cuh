@@ -119,6 +119,22 @@ __device__ __forceinline__ void tc_st_32x32b_x16(uint32_t taddr, const uint32_t 
     asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
 
+__device__ __forceinline__ void tc_st_32x32b_x8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};"
+        ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]),
+        "r"(v[6]), "r"(v[7])
+        : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 8 or 16 consecutive TMEM columns of the warp's lane quarter.
+template <int CW>
+__device__ __forceinline__ void tc_st_32x32b(uint32_t taddr, const uint32_t (&v)[CW]) {
+    static_assert(CW == 8 || CW == 16, "8 or 16 columns");
+    if constexpr (CW == 8) tc_st_32x32b_x8(taddr, v);
+    else tc_st_32x32b_x16(taddr, v);
+}
+
 __device__ __forceinline__ void tc_commit(uint32_t bar) {
     asm volatile(
         "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
