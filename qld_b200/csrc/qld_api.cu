@@ -1179,8 +1179,10 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
     if (nsites == 0) return QLD_OK;
     if (!text || !sites || !valid || !words || !bc || !snip_len || !keep)
         return set_err(c, QLD_ERR_INVALID, "NULL argument");
+    int max_len = 0;
     for (int i = 0; i < nsites; ++i) {
         const qld_vcf_site &v = sites[i];
+        if (v.len > max_len) max_len = v.len;
         if (v.off < 0 || v.len < 0 || (unsigned long long)v.off + (unsigned)v.len > text_bytes ||
             v.gt_pos < 0 || v.n_states < 0 || v.n_states > 4)
             return set_err(c, QLD_ERR_INVALID, "site %d lies outside the text or is malformed", i);
@@ -1190,7 +1192,7 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
     const int scratch_cap = K * 64;
     const size_t ns = (size_t)nsites;
     int rc;
-    if ((rc = ensure(c, c->vText, text_bytes ? text_bytes : 1)) ||
+    if ((rc = ensure(c, c->vText, (text_bytes + 16) / 16 * 16)) ||
         (rc = ensure(c, c->vSites, ns * sizeof(qld_vcf_site))) ||
         (rc = ensure(c, c->vValid, (size_t)nsamples)) || (rc = ensure(c, c->vSlash, ns * 8)) ||
         (rc = ensure(c, c->vRoff, ns * 8)) ||
@@ -1207,7 +1209,7 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
     const char *dtext = static_cast<const char *>(c->vText.p);
     const qld_vcf_site *dsites = static_cast<const qld_vcf_site *>(c->vSites.p);
     const uint8_t *dvalid = static_cast<const uint8_t *>(c->vValid.p);
-    // 1. count: random draws per site
+    // 1. sites without unphased genotypes packed; random draws the others need
     cudaError_t e = launch_vcf_sites(dtext, dsites, nsites, dvalid, nsamples, ploidy, K, nullptr,
                                      nullptr, static_cast<long long *>(c->vSlash.p),
                                      static_cast<char *>(c->vScratch.p), scratch_cap, ctas,
@@ -1215,7 +1217,7 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
                                      static_cast<uint32_t *>(c->vBc.p),
                                      static_cast<int *>(c->vLen.p),
                                      static_cast<uint8_t *>(c->vKeep.p),
-                                     static_cast<int *>(c->vErr.p), st);
+                                     static_cast<int *>(c->vErr.p), max_len, st);
     if (e != cudaSuccess)
         return set_err(c, QLD_ERR_CUDA, "VCF count launch failed: %s", cudaGetErrorString(e));
     std::vector<long long> slash(ns), roff(ns);
@@ -1230,22 +1232,28 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
         return set_err(c, QLD_ERR_INVALID,
                        "unphased genotypes need %lld random draws and no generator was given",
                        total);
-    std::vector<unsigned> rnd((size_t)(total > 0 ? total : 1));
+    std::vector<unsigned> rnd((size_t)total);
     for (long long i = 0; i < total; ++i) rnd[(size_t)i] = rng(rng_user);
-    if ((rc = ensure(c, c->vRnd, rnd.size() * 4))) return rc;
-    CUDA_TRY(c, cudaMemcpyAsync(c->vRnd.p, rnd.data(), rnd.size() * 4, cudaMemcpyHostToDevice, st));
-    CUDA_TRY(c, cudaMemcpyAsync(c->vRoff.p, roff.data(), ns * 8, cudaMemcpyHostToDevice, st));
-    // 2. pack
-    e = launch_vcf_sites(dtext, dsites, nsites, dvalid, nsamples, ploidy, K,
-                         static_cast<const unsigned *>(c->vRnd.p),
-                         static_cast<const long long *>(c->vRoff.p),
-                         static_cast<long long *>(c->vSlash.p), static_cast<char *>(c->vScratch.p),
-                         scratch_cap, ctas, static_cast<uint64_t *>(c->vWords.p),
-                         static_cast<uint32_t *>(c->vBc.p), static_cast<int *>(c->vLen.p),
-                         static_cast<uint8_t *>(c->vKeep.p), static_cast<int *>(c->vErr.p), st);
-    if (e != cudaSuccess)
-        return set_err(c, QLD_ERR_CUDA, "VCF pack launch failed: %s", cudaGetErrorString(e));
-    c->stats.kernel_launches += 2;
+    c->stats.kernel_launches++;
+    if (total > 0) {
+        if ((rc = ensure(c, c->vRnd, rnd.size() * 4))) return rc;
+        CUDA_TRY(c, cudaMemcpyAsync(c->vRnd.p, rnd.data(), rnd.size() * 4, cudaMemcpyHostToDevice,
+                                    st));
+        CUDA_TRY(c, cudaMemcpyAsync(c->vRoff.p, roff.data(), ns * 8, cudaMemcpyHostToDevice, st));
+        // 2. the sites with unphased genotypes
+        e = launch_vcf_sites(dtext, dsites, nsites, dvalid, nsamples, ploidy, K,
+                             static_cast<const unsigned *>(c->vRnd.p),
+                             static_cast<const long long *>(c->vRoff.p),
+                             static_cast<long long *>(c->vSlash.p),
+                             static_cast<char *>(c->vScratch.p), scratch_cap, ctas,
+                             static_cast<uint64_t *>(c->vWords.p),
+                             static_cast<uint32_t *>(c->vBc.p), static_cast<int *>(c->vLen.p),
+                             static_cast<uint8_t *>(c->vKeep.p), static_cast<int *>(c->vErr.p),
+                             max_len, st);
+        if (e != cudaSuccess)
+            return set_err(c, QLD_ERR_CUDA, "VCF pack launch failed: %s", cudaGetErrorString(e));
+        c->stats.kernel_launches++;
+    }
     std::vector<int> err(ns);
     CUDA_TRY(c, cudaMemcpyAsync(words, c->vWords.p, ns * K * 8, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(c, cudaMemcpyAsync(bc, c->vBc.p, ns * 4, cudaMemcpyDeviceToHost, st));

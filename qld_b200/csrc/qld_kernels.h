@@ -111,11 +111,13 @@ struct StatesParams {
 extern const int kStatesRows;   // B rows per tile
 cudaError_t launch_states(const StatesParams &p, int tiles_b, cudaStream_t st);
 
-// VCF sites -> packed rows (vcf_pack.cu).  With rnd_off NULL the launch only
-// counts: per site the random draws its unphased genotypes need
-// (slash_count), its row length and count-stage errors.  Otherwise it packs,
-// drawing site s's numbers from rnd[rnd_off[s]...].  Each CTA uses
-// scratch_cap bytes of scratch (>= K * 64).
+// VCF sites -> packed rows (vcf_pack.cu), in one launch or two.  The first
+// (rnd_off NULL) packs the sites without unphased genotypes and writes per site
+// the random draws the others need (slash_count) with their row length and
+// errors; the second packs those, drawing site s's numbers from
+// rnd[rnd_off[s]...].  Each CTA uses scratch_cap bytes of scratch (>= K * 64).
+// text is readable up to the next multiple of 16 bytes past its end; max_len
+// bounds the sites' len.
 enum VcfError {
     QLD_VCF_OK = 0,
     QLD_VCF_EMPTY_GT = 1,     // the GT subfield is empty
@@ -132,7 +134,7 @@ cudaError_t launch_vcf_sites(const char *text, const qld_vcf_site *sites, int ns
                              const unsigned *rnd, const long long *rnd_off,
                              long long *slash_count, char *scratch, int scratch_cap, int ctas,
                              uint64_t *words, uint32_t *bc, int *snip_len, uint8_t *keep,
-                             int *err, cudaStream_t st);
+                             int *err, int max_len, cudaStream_t st);
 
 // Report filter over `rows` r^2 rows (ldr >= m rounded up to 128 floats,
 // 16-byte aligned rows): mask (rows x W words, W = ceil(m / 32)), per-row
