@@ -351,13 +351,17 @@ __device__ __forceinline__ void tc_ld_32x32b(uint32_t taddr, uint32_t (&v)[CW]) 
     else tc_ld_32x32b_x32(taddr, v);
 }
 
+// Named barrier of whole warps.  bar.sync wants a warp's lanes to arrive
+// together, and a lane may still be in a branch of the caller's.
 __device__ __forceinline__ void named_bar_sync(int id, int nthreads) {
+    __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory");
 }
 
 // named_bar_sync that also tells every thread whether `x` held in any of them.
 __device__ __forceinline__ bool named_bar_or(int id, int nthreads, bool x) {
     uint32_t r;
+    __syncwarp();
     asm volatile(
         "{\n\t.reg .pred p, q;\n\t"
         "setp.ne.u32 p, %3, 0;\n\t"
