@@ -14,7 +14,7 @@
 // the MMAs fill the other, and each SM's shared memory supplies every
 // unpacked row once per MMA.
 //
-// Roles (both CTAs of a pair, 576 threads):
+// Roles (both CTAs of a pair, 576 or 608 threads):
 //   warp 0       TMA producer: the CTA's 128 A rows and 120 B rows, 8 packed
 //                words (512 samples) per stage, 64-byte swizzle.
 //   warp 1       TMEM allocation for the pair (cta_group::2); in rank 0 the
@@ -46,6 +46,10 @@
 //                23,000 cycles a tile's epilogue took.  Twelve epilogue warps
 //                (80 registers): band of 1,000 210 us against 199, reference
 //                mode 347 against 341.
+//   warp 18      (FW) the column factors, a tile or two ahead: the epilogue
+//                warps then neither divide for columns nor meet at a barrier,
+//                and each runs ahead of the others by up to a tile.  Where it
+//                pays: factor_warp() below.
 // Every wait is bounded.  No thread returns early: both CTAs meet at the
 // cluster barriers at start and end on every path, including after a
 // timeout, and the TMEM is released only after the last MMA has completed.
@@ -76,8 +80,8 @@ constexpr int GROUPS = 4, GROUP_WARPS = 2;
 constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS, EPI_WARPS = 8;
 constexpr int FIRST_UNPACK_WARP = 2;
 constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
-constexpr int EPILOGUE = EPI_WARPS * 32;
-constexpr int THREADS = (FIRST_EPI_WARP + EPI_WARPS) * 32;   // 576
+constexpr int FACTOR_WARP = FIRST_EPI_WARP + EPI_WARPS;
+constexpr int threads(bool fw) { return (FACTOR_WARP + fw) * 32; }   // 576 or 608
 constexpr int GROUP_THREADS = GROUP_WARPS * 32;              // unpackers per stage
 constexpr int TASKS = (HM + HN + GROUP_THREADS - 1) / GROUP_THREADS;   // rows per thread
 constexpr uint32_t TMEM_COLS = 512;
@@ -98,8 +102,8 @@ struct Smem {
     static constexpr int OFF_ROWS = OFF_P + PST * P_BYTES;
     static constexpr int ROWS_BYTES = COLS_N * (MODE == R2_EXACT ? 8 : epi::COLR_BYTES);
     static constexpr int OFF_BAR = OFF_ROWS + 2 * ROWS_BYTES;   // this tile's and the next one's
-    static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1;
-    static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;
+    static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1 + 2 + 2;
+    static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;        // and the halves' special flags
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
     static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
@@ -110,7 +114,7 @@ struct Smem {
     static_assert(PST * SUB % GROUPS == 0 && GROUPS <= UST, "stage rings");
 };
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
-static_assert(SUB == 2 && EPILOGUE >= COLS_N && EPI_WARPS % 4 == 0, "work split");
+static_assert(SUB == 2 && EPI_WARPS * 32 == COLS_N && EPI_WARPS == 8, "work split");
 
 // BAND: a band's launch (its window and tiles); otherwise two regions or a
 // single region.  One kernel for both ran the other two 1.2 % slower.
@@ -121,8 +125,10 @@ static_assert(SUB == 2 && EPILOGUE >= COLS_N && EPI_WARPS % 4 == 0, "work split"
 // 1,920 samples 22.0 -> 18.0 us, 12,000 x 5,120 155 -> 141, band of 1,000 over
 // 50,000 x 10,001 199 -> 192, in reference mode 241 -> 222.  A branch in one
 // kernel cost the launches with counts 1 %.
-template <int MODE, bool BAND, bool FULL, bool PLAIN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
+// FW: a warp of its own stores the column factors (otherwise the epilogue warps
+// do, after a tile's chunks; pair_factor_warp chooses).
+template <int MODE, bool BAND, bool FULL, bool PLAIN, bool FW>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads(FW), 1)
 k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                const LdParams p, const RowTiles all, const int ntiles) {
     using L = Smem<MODE>;
@@ -136,7 +142,9 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     uint64_t *accfull = bars + 2 * PST + 2 * UST;
     uint64_t *accempty = accfull + 2;
     uint64_t *mma_done = accempty + 2;
+    uint64_t *facfull = mma_done + 1, *facempty = facfull + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM);
+    volatile uint32_t *col_flag = tmem_slot + 1;     // a column of the half is special
 
     const uint32_t rank = cluster_rank();
     const int pair = (int)cluster_id_x(), npairs = (int)cluster_count_x();
@@ -164,6 +172,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         for (int b = 0; b < 2; ++b) {
             mbar_init(smem_u32(&accfull[b]), 1);
             mbar_init(smem_u32(&accempty[b]), 2 * EPI_WARPS);   // both CTAs' epilogues
+            mbar_init(smem_u32(&facfull[b]), 1);
+            mbar_init(smem_u32(&facempty[b]), EPI_WARPS);
         }
         mbar_init(smem_u32(mma_done), 1);
         fence_barrier_init();
@@ -299,15 +309,50 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 mbar_arrive(smem_u32(&pempty[ps]));     // one group per sub-stage
             }
         }
+    } else if (FW && warp == FACTOR_WARP) {
+        // ------------------------------------------------- column factors --
+        int cur_t = 0, cur_base = 0;
+        for (int it = 0; it < my_tiles; ++it) {
+            const int ab = it & 1;
+            int a_row, b_row;
+            tl.decode_from(pair + it * npairs, a_row, b_row, cur_t, cur_base);
+            // every column factor the chunks read; 0 past the tile and the task
+            uint32_t cb[COLS_N / 32];
+#pragma unroll
+            for (int i = 0; i < COLS_N / 32; ++i) {
+                const int e = i * 32 + lane;
+                cb[i] = e < bn && b_row + e < p.n ? p.bcB[b_row + e] : 0u;
+            }
+            const bool free = it < 2 || mbar_wait(smem_u32(&facempty[ab]), ((it >> 1) - 1) & 1,
+                                                  p.timeout_cycles, p.status);
+            if (!__all_sync(0xffffffffu, free)) {
+                if (lane == 0) flag_error(p.status, ST_TIMEOUT_EMPTY);
+                break;
+            }
+            uint8_t *base = smem + L::OFF_ROWS + ab * L::ROWS_BYTES;
+            bool special = false;
+#pragma unroll
+            for (int i = 0; i < COLS_N / 32; ++i) {
+                if constexpr (MODE == R2_EXACT)
+                    special |= epi::store_col_f32(epi::ColsF(base, COLS_N), i * 32 + lane, cb[i], p.S);
+                else
+                    special |= epi::store_col_ref(epi::ColsR2(base, COLS_N), i * 32 + lane, cb[i],
+                                                  p.S);
+            }
+            special = __any_sync(0xffffffffu, special);   // and every lane's factors are stored
+            if (lane == 0) {
+                col_flag[ab] = special;
+                mbar_arrive(smem_u32(&facfull[ab]));
+            }
+            __syncwarp();
+        }
     } else {
         // ------------------------------------------------------- epilogue --
         // The bit counts of the next tile's rows are loaded while this tile is
-        // worked on, and its factors stored in the other half of the buffer.
+        // worked on, and (!FW) its factors stored in the other half of the buffer.
         const int et = tid - FIRST_EPI_WARP * 32;
         const int ew = warp - FIRST_EPI_WARP;
         const int q = warp & 3;                 // TMEM lane quarter
-        const int colh = ew >> 2;               // chunks colh, colh + EPI_WARPS / 4, ... (< 15)
-        bool failed = false;
         int cur_t = 0, cur_base = 0, a_row = 0, b_row = 0;
         uint32_t ca = 0, cb = 0;                // bit counts of my row and column
         auto load_counts = [&](int it) {
@@ -315,20 +360,19 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int a = a_row + (int)rank * HM + q * 32 + lane, b = b_row + et;
             ca = a < p.m ? p.bcA[a] : 0u;
             // every column factor the chunks read; 0 past the tile and the task
-            cb = et < bn && b < p.n ? p.bcB[b] : 0u;
+            if (!FW) cb = et < bn && b < p.n ? p.bcB[b] : 0u;
         };
+        bool failed = false, special = false;
         epi::ARowR ra{};
         epi::ARowF raf{};
-        bool special = false;
         auto store_factors = [&](int it) {
             uint8_t *base = smem + L::OFF_ROWS + (it & 1) * L::ROWS_BYTES;
             if constexpr (MODE == R2_EXACT) {
                 raf = epi::make_arow_f32(ca, p.S);
-                special = et < COLS_N && epi::store_col_f32(epi::ColsF(base, COLS_N), et, cb, p.S);
+                if (!FW) special = epi::store_col_f32(epi::ColsF(base, COLS_N), et, cb, p.S);
             } else {
                 ra = epi::make_arow_ref(ca, p.S);
-                special = et < COLS_N &&
-                          epi::store_col_ref(epi::ColsR2(base, COLS_N), et, cb, p.S);
+                if (!FW) special = epi::store_col_ref(epi::ColsR2(base, COLS_N), et, cb, p.S);
             }
         };
         if (my_tiles > 0) {
@@ -337,17 +381,27 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         for (int it = 0; it < my_tiles; ++it) {
             const int ab = it & 1;
+            // chunks colh, colh + 2, ... of the 15: without a barrier, 8 and 7 in turn
+            const int colh = (ew >> 2) ^ (FW ? ab : 0);
             const int a = a_row + (int)rank * HM + q * 32 + lane, b_tile = b_row;
             const bool a_ok = a < p.m;
-            // this tile's factors are stored, and the other half is free
-            const bool cols_special = named_bar_or(1, EPILOGUE, special);
+            // this tile's factors are stored, and (!FW) the other half is free
+            bool cols_special = false;
+            if constexpr (!FW) cols_special = named_bar_or(1, EPI_WARPS * 32, special);
             if (it + 1 < my_tiles) load_counts(it + 1);
-            bool ready = !failed && mbar_wait(smem_u32(&accfull[ab]), (it >> 1) & 1,
-                                              p.timeout_cycles, p.status);
+            bool ready = !failed &&
+                         (!FW || mbar_wait(smem_u32(&facfull[ab]), (it >> 1) & 1,
+                                           p.timeout_cycles, p.status)) &&
+                         mbar_wait(smem_u32(&accfull[ab]), (it >> 1) & 1, p.timeout_cycles,
+                                   p.status);
             ready = __all_sync(0xffffffffu, ready);
-            if (!ready && !failed) {
+            if (!ready && !failed) {            // (!FW: keep meeting the others at the barrier)
                 if (lane == 0) flag_error(p.status, ST_TIMEOUT_MMA);
                 failed = true;
+            }
+            if constexpr (FW) {
+                if (!ready) break;
+                cols_special = col_flag[ab] != 0u;
             }
             if (ready) {
                 __syncwarp();
@@ -406,7 +460,10 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                 }
                 tc_fence_before();
                 __syncwarp();
-                if (lane == 0) mbar_arrive_rank(smem_u32(&accempty[ab]), 0);
+                if (lane == 0) {
+                    mbar_arrive_rank(smem_u32(&accempty[ab]), 0);
+                    if (FW) mbar_arrive(smem_u32(&facempty[ab]));
+                }
             }
             if (it + 1 < my_tiles) store_factors(it + 1);
         }
@@ -435,14 +492,14 @@ int max_pairs() {
     static std::atomic<int> known;
     int n = known.load(std::memory_order_relaxed);
     if (n > 0) return n;
-    auto kern = k_ld_mxf4_pair<R2_EXACT, false, true, true>;
+    auto kern = k_ld_mxf4_pair<R2_EXACT, false, true, true, true>;
     int dev = 0, sms = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
         return 1;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * (sms / 2), 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.blockDim = dim3(threads(true), 1, 1);
     cfg.dynamicSmemBytes = Smem<R2_EXACT>::BYTES;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Smem<R2_EXACT>::BYTES) != cudaSuccess ||
@@ -454,10 +511,10 @@ int max_pairs() {
     return n;
 }
 
-template <int MODE, bool BAND, bool FULL, bool PLAIN>
+template <int MODE, bool BAND, bool FULL, bool PLAIN, bool FW>
 cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                         const RowTiles &tl, cudaStream_t st) {
-    auto kern = k_ld_mxf4_pair<MODE, BAND, FULL, PLAIN>;
+    auto kern = k_ld_mxf4_pair<MODE, BAND, FULL, PLAIN, FW>;
     static std::atomic<unsigned long long> allowed;
     cudaError_t e = allow_smem(kern, Smem<MODE>::BYTES, allowed);
     if (e != cudaSuccess) return e;
@@ -467,7 +524,7 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     cudaLaunchAttribute at = overlap_attr();
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(2 * pairs), 1, 1);
-    cfg.blockDim = dim3(THREADS, 1, 1);
+    cfg.blockDim = dim3(threads(FW), 1, 1);
     cfg.dynamicSmemBytes = Smem<MODE>::BYTES;
     cfg.stream = st;
     cfg.attrs = &at;
@@ -475,14 +532,21 @@ cudaError_t launch_mode(const CUtensorMap &tmA, const CUtensorMap &tmB, const Ld
     return cudaLaunchKernelEx(&cfg, kern, tmA, tmB, p, tl, ntiles);
 }
 
-template <int MODE, bool PLAIN>
+template <int MODE, bool PLAIN, bool FW>
 cudaError_t launch_tiles(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                          const RowTiles &tl, cudaStream_t st) {
     if (tl.band > 0)
-        return tl.bn == BN ? launch_mode<MODE, true, true, PLAIN>(tmA, tmB, p, tl, st)
-                           : launch_mode<MODE, true, false, PLAIN>(tmA, tmB, p, tl, st);
-    return tl.bn == BN ? launch_mode<MODE, false, true, PLAIN>(tmA, tmB, p, tl, st)
-                       : launch_mode<MODE, false, false, PLAIN>(tmA, tmB, p, tl, st);
+        return tl.bn == BN ? launch_mode<MODE, true, true, PLAIN, FW>(tmA, tmB, p, tl, st)
+                           : launch_mode<MODE, true, false, PLAIN, FW>(tmA, tmB, p, tl, st);
+    return tl.bn == BN ? launch_mode<MODE, false, true, PLAIN, FW>(tmA, tmB, p, tl, st)
+                       : launch_mode<MODE, false, false, PLAIN, FW>(tmA, tmB, p, tl, st);
+}
+
+template <int MODE, bool PLAIN>
+cudaError_t launch_rule(bool fw, const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
+                        const RowTiles &tl, cudaStream_t st) {
+    return fw ? launch_tiles<MODE, PLAIN, true>(tmA, tmB, p, tl, st)
+              : launch_tiles<MODE, PLAIN, false>(tmA, tmB, p, tl, st);
 }
 
 }  // namespace
@@ -529,14 +593,30 @@ int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
     return bn;
 }
 
+// Whether the column factors get a warp of their own.  The epilogue warps pay
+// ~2,000 cycles a tile for loading and dividing them and meeting at a barrier,
+// which is the launch's time where its epilogues are (few stages per tile) and
+// hidden behind the MMAs elsewhere; there the extra warp costs 1-4 % (whatever
+// warps it shares a scheduler with unpack later, and a stage waits for both
+// CTAs' slowest).  Exact mode, K = 60 / 80 / 100 / 120 / 140: 9,001 x 7,003
+// 114 -> 102, 128 -> 117, 147 -> 144, 161 -> 161, 185 -> 188 us; reference
+// mode, K = 80 / 120 / 160 / 200 / 260: 195 -> 164, 210 -> 184, 231 -> 221,
+// 265 -> 266, 327 -> 339; 12,000 SNPs, K = 80: 144 -> 132, 222 -> 187.
+// A launch of one or two waves gains less than the first tile's factors, all
+// from one warp, cost it: 3,300 SNPs, exact mode, K = 60 17.6 -> 17.8.
+bool factor_warp(const RowTiles &tl, int K, int r2_mode) {
+    return K <= (r2_mode == R2_REFERENCE ? 160 : 100) && tl.count() > 2 * max_pairs();
+}
+
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              const RowTiles &tl, int r2_mode, cudaStream_t st) {
+    const bool fw = factor_warp(tl, p.K, r2_mode);
     if (r2_mode == R2_REFERENCE)
         return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
-                   ? launch_tiles<R2_REFERENCE, true>(tmA, tmB, p, tl, st)
-                   : launch_tiles<R2_REFERENCE, false>(tmA, tmB, p, tl, st);
-    return !p.counts ? launch_tiles<R2_EXACT, true>(tmA, tmB, p, tl, st)
-                     : launch_tiles<R2_EXACT, false>(tmA, tmB, p, tl, st);
+                   ? launch_rule<R2_REFERENCE, true>(fw, tmA, tmB, p, tl, st)
+                   : launch_rule<R2_REFERENCE, false>(fw, tmA, tmB, p, tl, st);
+    return !p.counts ? launch_rule<R2_EXACT, true>(fw, tmA, tmB, p, tl, st)
+                     : launch_rule<R2_EXACT, false>(fw, tmA, tmB, p, tl, st);
 }
 
 }  // namespace qld
