@@ -28,11 +28,14 @@
 // throughout, 300 tasks of 64-2,048 SNPs took 567 us against 533 (reference
 // mode 647 / 614).
 //
-// Roles per CTA (608 threads in R2_EXACT, 736 in R2_REFERENCE): warp 0 TMA of
-// the CTA's rows, warp 1 TMEM and (rank 0) the MMAs,
-// warps 2-9 unpack in four groups taking the 256-sample stages in turn (each
-// thread whole rows), warps 10-17 (10-21) epilogue, two (three) per TMEM lane
-// quarter, the last warp (rank 0) the queue.  TMEM: two accumulators
+// Roles per CTA (640 threads): warp 0 TMA of the CTA's rows, warp 1 TMEM and
+// (rank 0) the MMAs, warps 2-9 unpack in four groups taking the 256-sample
+// stages in turn (each thread whole rows), warps 10-17 epilogue, two per TMEM
+// lane quarter, warp 18 (rank 0) the queue, warp 19 the column factors, an item
+// ahead of the epilogue.  With the factors loaded, divided and handed over at
+// two barriers by the epilogue warps themselves, which items of few stages or
+// rows pay in full, the 300 tasks took 488 us against 472 (reference mode, then
+// with twelve epilogue warps, 588 against 549).  TMEM: two accumulators
 // (columns 0 and 256), so a tile's epilogue overlaps the next tile's MMAs,
 // and the scale factors at columns 496-511.  Every wait is bounded and no
 // thread returns early: both CTAs meet at the cluster barriers at start and
@@ -56,7 +59,7 @@ constexpr int SUB = 2;                      // unpacked stages (256 samples) per
 constexpr int UST = 4;                      // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;       // 8 KB
 constexpr int P_MAX = (HM + HN) * PW * 8;   // up to 15.5 KB delivered per stage
-constexpr int P_BYTES = 16384;              // stage stride: A rows, then B rows
+constexpr int P_BYTES = 15872;              // stage stride: A rows, then B rows (a multiple of 512)
 constexpr int UA_BYTES = HM * 128;          // 16 KB: 256 E2M1 per row
 constexpr int U_BYTES = (HM + HN) * 128;    // 31 KB: A rows, then B rows
 constexpr int GROUPS = 4, GROUP_WARPS = 2;  // as ld_mxf4_pair.cu
@@ -64,6 +67,12 @@ constexpr int UNPACK_WARPS = GROUPS * GROUP_WARPS;
 constexpr int GROUP_THREADS = GROUP_WARPS * 32;
 constexpr int FIRST_UNPACK_WARP = 2;
 constexpr int FIRST_EPI_WARP = FIRST_UNPACK_WARP + UNPACK_WARPS;
+// Twelve epilogue warps (at 80 registers): 300-task mix 492 us against 472,
+// reference mode 552 against 549.
+constexpr int EPI_WARPS = 8;
+constexpr int QUEUE_WARP = FIRST_EPI_WARP + EPI_WARPS;
+constexpr int FACTOR_WARP = QUEUE_WARP + 1;
+constexpr int THREADS = (FACTOR_WARP + 1) * 32;              // 640
 constexpr int TASKS = (HM + HN + GROUP_THREADS - 1) / GROUP_THREADS;   // rows per thread
 constexpr uint32_t TMEM_COLS = 512;
 constexpr uint32_t ACC_STRIDE = 256;
@@ -72,22 +81,8 @@ constexpr int COLS_N = 256;                                  // epilogue column 
 constexpr uint16_t BOTH = 0x3;                               // CTA mask of a commit to both ranks
 constexpr int QSLOTS = 4;                                    // item ring depth
 // arrivals on rank 0's slot-free barrier per item: rank 0's MMA warp; both
-// CTAs' TMA threads, unpack and epilogue warps
-// Epilogue warps per r^2 mode: eight in R2_EXACT, twelve in R2_REFERENCE,
-// whose longer per-pair sequence leaves items below ~6,000 samples waiting
-// on their epilogue (300-task mix, one-column arithmetic: 689 us against 706
-// with eight; exact mode with twelve: 574 against 566, at the 80 registers 704
-// threads leave).  Popping the next item early to prefetch its factors, as
-// ld_mxf4_pair.cu does for its fixed tile list, costs 3 % here: 584.
-template <int MODE>
-struct Roles {
-    static constexpr int EPI_WARPS = MODE == R2_REFERENCE ? 12 : 8;
-    static constexpr int EPI_THREADS = EPI_WARPS * 32;
-    static constexpr int QUEUE_WARP = FIRST_EPI_WARP + EPI_WARPS;
-    static constexpr int THREADS = (QUEUE_WARP + 1) * 32;               // 608 or 736
-    static constexpr int ITEM_USERS = 2 * (1 + UNPACK_WARPS + EPI_WARPS) + 1;
-    static_assert(EPI_WARPS % 4 == 0 && EPI_THREADS >= COLS_N, "epilogue split");
-};
+// CTAs' TMA threads, unpack, epilogue and factor warps
+constexpr int ITEM_USERS = 2 * (1 + UNPACK_WARPS + EPI_WARPS + 1) + 1;
 
 // Shared-memory layout per r^2 mode: R2_EXACT needs 8 bytes of column
 // factors per column (epi::ColsF), R2_REFERENCE 16 (epi::ColsR); both leave
@@ -99,21 +94,21 @@ struct Smem {
     static constexpr int OFF_P = OFF_U + UST * U_BYTES;
     static constexpr int OFF_ROWS = OFF_P + PST * P_BYTES;
     static constexpr int ROWS_BYTES = COLS_N * (MODE == R2_EXACT ? 8 : epi::COLR_BYTES);
-    static constexpr int OFF_ITEMS = OFF_ROWS + ROWS_BYTES;
+    static constexpr int OFF_ITEMS = OFF_ROWS + 2 * ROWS_BYTES;   // two items' factors
     static constexpr int OFF_BAR = OFF_ITEMS + QSLOTS * 16;
-    static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1 + 2 * QSLOTS;
-    static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;
+    static constexpr int NBARS = 2 * PST + 2 * UST + 2 + 2 + 1 + 2 * QSLOTS + 2 + 2;
+    static constexpr int OFF_TMEM = OFF_BAR + NBARS * 8;        // and the halves' special flags
     static constexpr int BYTES = OFF_TMEM + 16 + 1024;
     static_assert(BYTES <= 232448, "shared memory budget");
     static_assert(U_BYTES % 1024 == 0 && UA_BYTES % 1024 == 0 && OFF_P % 1024 == 0 &&
-                      P_MAX <= P_BYTES && OFF_ITEMS % 16 == 0,
-                  "swizzled stages must start on 1024-byte boundaries");
+                      P_BYTES % 512 == 0 && P_MAX <= P_BYTES && OFF_ITEMS % 16 == 0,
+                  "swizzled stages must start on whole swizzle atoms");
     // group g takes sub-stage g % 2 of packed stages g / 2, g / 2 + 2, ...: a
     // slot always belongs to the same two groups
     static_assert(PST % 2 == 0 && GROUPS == 2 * SUB && GROUPS <= UST, "stage rings");
 };
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
-static_assert(SUB == 2, "work split");
+static_assert(SUB == 2 && EPI_WARPS % 4 == 0, "work split");
 
 // A work item: task (< 0: end of the queue), its tile's first A and B row, and
 // the packed stages (low 24 bits) and tile rows / 16 (high 8) of the task.
@@ -166,10 +161,9 @@ struct JobFields {
 // PLAIN: no task has counts or a summary (in reference mode: every S within
 // R2_PLAIN_S..2^24), as ld_mxf4_pair.cu's.
 template <int MODE, bool PLAIN>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Roles<MODE>::THREADS, 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1)
 k_ld_batch(const BatchParams bp) {
     using L = Smem<MODE>;
-    using R = Roles<MODE>;
     constexpr int PST = L::PST;
     extern __shared__ uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>(
@@ -181,10 +175,10 @@ k_ld_batch(const BatchParams bp) {
     uint64_t *accempty = accfull + 2;
     uint64_t *mma_done = accempty + 2;
     uint64_t *ifull = mma_done + 1, *iempty = ifull + QSLOTS;
+    uint64_t *facfull = iempty + QSLOTS, *facempty = facfull + 2;
     Item *items = reinterpret_cast<Item *>(smem + L::OFF_ITEMS);
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM);
-    const epi::ColsR2 colsr(smem + L::OFF_ROWS, COLS_N);   // R2_REFERENCE factors
-    const epi::ColsF colsf(smem + L::OFF_ROWS, COLS_N);   // R2_EXACT: FP32 factors
+    volatile uint32_t *col_flag = tmem_slot + 1;     // a column of the half is special
 
     const uint32_t rank = cluster_rank();
     const int tid = threadIdx.x;
@@ -210,12 +204,14 @@ k_ld_batch(const BatchParams bp) {
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(smem_u32(&accfull[s]), 1);
-            mbar_init(smem_u32(&accempty[s]), 2 * R::EPI_WARPS);   // both CTAs' epilogues
+            mbar_init(smem_u32(&accempty[s]), 2 * EPI_WARPS);   // both CTAs' epilogues
+            mbar_init(smem_u32(&facfull[s]), 1);
+            mbar_init(smem_u32(&facempty[s]), EPI_WARPS);
         }
         mbar_init(smem_u32(mma_done), 1);
         for (int s = 0; s < QSLOTS; ++s) {
             mbar_init(smem_u32(&ifull[s]), 1);
-            mbar_init(smem_u32(&iempty[s]), R::ITEM_USERS);
+            mbar_init(smem_u32(&iempty[s]), ITEM_USERS);
         }
         fence_barrier_init();
     }
@@ -235,7 +231,7 @@ k_ld_batch(const BatchParams bp) {
     cluster_sync_all();
     tc_fence_after();
 
-    if (warp == R::QUEUE_WARP) {
+    if (warp == QUEUE_WARP) {
         // ------------------------------------------- work queue (rank 0) --
         if (rank == 0) {
             bool ok = true;
@@ -409,117 +405,142 @@ k_ld_batch(const BatchParams bp) {
             __syncwarp();
             if (lane == 0) release_item(qi);
         }
-    } else {
-        // ------------------------------------------------------- epilogue --
-        // The epilogue warps meet at named barriers, so they must leave the
-        // loop together: a failure is recorded in a shared flag that is only
-        // read right after the first barrier of an item (every write to it
-        // happens before that barrier or between the second and third).
-        volatile int *epi_fail = reinterpret_cast<volatile int *>(smem + L::OFF_TMEM + 8);
-        const int et = tid - FIRST_EPI_WARP * 32;
-        const int ew = warp - FIRST_EPI_WARP;
-        const int q = warp & 3;             // TMEM lane quarter
-        const int colh = ew >> 2;           // chunks colh, colh + EPI_WARPS / 4, ...
-        if (et == 0) *epi_fail = 0;
-        named_bar_sync(1, R::EPI_THREADS);
+    } else if (warp == FACTOR_WARP) {
+        // ------------------------------------------------- column factors --
         for (int qi = 0;; ++qi) {
-            const bool got_item = wait_item(qi);
-            if (!__all_sync(0xffffffffu, got_item) && lane == 0) {
-                flag_error(bp.status, ST_TIMEOUT_FULL);
-                *epi_fail = 1;
+            const int ab = qi & 1;
+            if (!__all_sync(0xffffffffu, wait_item(qi))) {
+                if (lane == 0) flag_error(bp.status, ST_TIMEOUT_FULL);
+                break;
             }
             const Item it = items[qi % QSLOTS];
-            named_bar_sync(1, R::EPI_THREADS);
-            if (*epi_fail || it.job < 0) break;
+            if (it.job < 0) break;
+            const BatchJob &J = bp.jobs[it.job];
+            const int n = J.n, S = J.S;
+            // every column factor the chunks read; 0 past the tile and the task
+            uint32_t cb[COLS_N / 32];
+#pragma unroll
+            for (int i = 0; i < COLS_N / 32; ++i) {
+                const int e = i * 32 + lane;
+                cb[i] = e < it.bn() && it.b_row + e < n ? J.bcB[it.b_row + e] : 0u;
+            }
+            const bool free = qi < 2 || mbar_wait(smem_u32(&facempty[ab]), ((qi >> 1) - 1) & 1,
+                                                  limit, bp.status);
+            if (!__all_sync(0xffffffffu, free)) {
+                if (lane == 0) flag_error(bp.status, ST_TIMEOUT_EMPTY);
+                break;
+            }
+            uint8_t *base = smem + L::OFF_ROWS + ab * L::ROWS_BYTES;
+            bool special = false;
+#pragma unroll
+            for (int i = 0; i < COLS_N / 32; ++i) {
+                if constexpr (MODE == R2_EXACT)
+                    special |= epi::store_col_f32(epi::ColsF(base, COLS_N), i * 32 + lane, cb[i], S);
+                else
+                    special |= epi::store_col_ref(epi::ColsR2(base, COLS_N), i * 32 + lane, cb[i], S);
+            }
+            special = __any_sync(0xffffffffu, special);   // and every lane's factors are stored
+            if (lane == 0) {
+                col_flag[ab] = special;
+                mbar_arrive(smem_u32(&facfull[ab]));
+                release_item(qi);
+            }
+            __syncwarp();
+        }
+    } else {
+        // ------------------------------------------------------- epilogue --
+        const int ew = warp - FIRST_EPI_WARP;
+        const int q = warp & 3;             // TMEM lane quarter
+        for (int qi = 0;; ++qi) {
+            if (!__all_sync(0xffffffffu, wait_item(qi))) {
+                if (lane == 0) flag_error(bp.status, ST_TIMEOUT_FULL);
+                break;
+            }
+            const Item it = items[qi % QSLOTS];
+            if (it.job < 0) break;
             const JobFields J(bp.jobs[it.job]);
             const int ab = qi & 1;
+            // chunks colh, colh + EPI_WARPS / 4, ...: the longer shares in turn
+            const int colh = ((ew >> 2) + qi) % (EPI_WARPS / 4);
             const int a = it.a_row + (int)rank * HM + q * 32 + lane;
             const bool a_ok = a < J.m;
             const uint32_t ca = a_ok ? J.bcA[a] : 0u;
-            bool special = false;
-            if (et < COLS_N) {   // every column factor the chunks read; 0 past the tile and the task
-                const int b = it.b_row + et;
-                const uint32_t cb = (et < it.bn() && b < J.n) ? J.bcB[b] : 0u;
-                if constexpr (MODE == R2_EXACT)
-                    special = epi::store_col_f32(colsf, et, cb, J.S);
-                else
-                    special = epi::store_col_ref(colsr, et, cb, J.S);
+            const epi::ARowR ra = epi::make_arow_ref(ca, J.S);
+            const epi::ARowF raf = epi::make_arow_f32(ca, J.S);
+            const bool ready = mbar_wait(smem_u32(&facfull[ab]), (qi >> 1) & 1, limit, bp.status) &&
+                               mbar_wait(smem_u32(&accfull[ab]), (qi >> 1) & 1, limit, bp.status);
+            if (!__all_sync(0xffffffffu, ready)) {
+                if (lane == 0) flag_error(bp.status, ST_TIMEOUT_MMA);
+                break;
             }
-            const bool cols_special = named_bar_or(1, R::EPI_THREADS, special);
-            bool ready = mbar_wait(smem_u32(&accfull[ab]), (qi >> 1) & 1, limit, bp.status);
-            ready = __all_sync(0xffffffffu, ready);
-            if (!ready) {
-                if (lane == 0) {
-                    flag_error(bp.status, ST_TIMEOUT_MMA);
-                    *epi_fail = 1;
-                }
-            } else {
-                __syncwarp();
-                tc_fence_after();
-                const epi::ARowR ra = epi::make_arow_ref(ca, J.S);
-                const epi::ARowF raf = epi::make_arow_f32(ca, J.S);
-                const uint32_t tbase =
-                    tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
-                const int n_tile = it.b_row + it.bn() < J.n ? it.b_row + it.bn() : J.n;
-                const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
-                epi::SumAcc acc;
-                // Chunks of 16 columns, in reference mode of 8 (more columns spill:
-                // 32 in exact mode 620 us against 566 on 300 tasks, 16 in
-                // reference mode 668 against 647)
-                constexpr int CW = MODE == R2_EXACT ? 16 : 8;
-                bool full = true;                // chunks with the rare cases' bookkeeping
-                if constexpr (PLAIN) {
-                    full = cols_special ||
-                           __any_sync(0xffffffffu, MODE == R2_EXACT ? raf.special : ra.k.y != ra.k.y);
-                    const long long step = (long long)(CW * R::EPI_WARPS / 4) * J.ldr;
-                    float *o = J.r2 + (long long)(it.b_row + colh * CW) * J.ldr + a;
-                    float rmax = 0.0f;
+            const bool cols_special = col_flag[ab] != 0u;
+            const epi::ColsR2 colsr(smem + L::OFF_ROWS + ab * L::ROWS_BYTES, COLS_N);
+            const epi::ColsF colsf(smem + L::OFF_ROWS + ab * L::ROWS_BYTES, COLS_N);
+            __syncwarp();
+            tc_fence_after();
+            const uint32_t tbase =
+                tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
+            const int n_tile = it.b_row + it.bn() < J.n ? it.b_row + it.bn() : J.n;
+            const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
+            epi::SumAcc acc;
+            // Chunks of 16 columns, in reference mode of 8 (more columns spill:
+            // 32 in exact mode 620 us against 566 on 300 tasks, 16 in
+            // reference mode 668 against 647)
+            constexpr int CW = MODE == R2_EXACT ? 16 : 8;
+            bool full = true;                // chunks with the rare cases' bookkeeping
+            if constexpr (PLAIN) {
+                full = cols_special ||
+                       __any_sync(0xffffffffu, MODE == R2_EXACT ? raf.special : ra.k.y != ra.k.y);
+                const long long step = (long long)(CW * EPI_WARPS / 4) * J.ldr;
+                float *o = J.r2 + (long long)(it.b_row + colh * CW) * J.ldr + a;
+                float rmax = 0.0f;
 #pragma unroll 1
-                    for (int c = colh; !full && c < it.bn() / CW; c += R::EPI_WARPS / 4, o += step) {
-                        const uint32_t taddr = tbase + (uint32_t)(c * CW);
-                        uint32_t v[CW];
-                        __syncwarp();
-                        tc_ld_32x32b<CW>(taddr, v);
-                        if constexpr (MODE == R2_EXACT)
-                            epi::chunk_f32_plain<CW>(v, raf, colsf, c * CW, it.b_row + c * CW, a,
-                                                     a_ok, n_tile, dlo, dhi, o, J.ldr, (float)J.S,
-                                                     rmax);
-                        else
-                            epi::chunk_ref_plain<CW>(
-                                v, ra, colsr, c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi,
-                                J.r2, o, J.ldr, 0, J.S,
-                                [&](uint32_t (&w)[CW]) { tc_ld_32x32b<CW>(taddr, w); });
-                    }
-                    if (MODE == R2_EXACT && __any_sync(0xffffffffu, rmax > epi::R2_RECHECK))
-                        full = true;
-                }
-#pragma unroll 1
-                for (int c = colh; full && c < it.bn() / CW; c += R::EPI_WARPS / 4) {   // the tile's chunks
+                for (int c = colh; !full && c < it.bn() / CW; c += EPI_WARPS / 4, o += step) {
+                    const uint32_t taddr = tbase + (uint32_t)(c * CW);
                     uint32_t v[CW];
                     __syncwarp();
-                    tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
-                    if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
-                                           c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
-                                           J.ldr, J.counts, J.ldc, 0, J.S);
-                        if (J.summary)
-                            acc.fold(v, it.b_row + c * CW, a, a_ok, J.n, J.symmetric,
-                                     J.threshold);
-                    } else {
-                        // the F32 accumulators hold the counts as floats
-                        epi::chunk_ref<0, true, CW>(v, ra, colsr, c * CW, it.b_row + c * CW, a,
-                                                    a_ok, n_tile, dlo, dhi, J.r2, J.ldr,
-                                                    J.counts, J.ldc, 0, J.S);
-                    }
+                    tc_ld_32x32b<CW>(taddr, v);
+                    if constexpr (MODE == R2_EXACT)
+                        epi::chunk_f32_plain<CW>(v, raf, colsf, c * CW, it.b_row + c * CW, a,
+                                                 a_ok, n_tile, dlo, dhi, o, J.ldr, (float)J.S,
+                                                 rmax);
+                    else
+                        epi::chunk_ref_plain<CW>(
+                            v, ra, colsr, c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi,
+                            J.r2, o, J.ldr, 0, J.S,
+                            [&](uint32_t (&w)[CW]) { tc_ld_32x32b<CW>(taddr, w); });
                 }
-                tc_fence_before();
-                __syncwarp();
-                if (lane == 0) mbar_arrive_rank(smem_u32(&accempty[ab]), 0);
-                if (MODE == R2_EXACT && J.summary) acc.flush(J.summary);
+                if (MODE == R2_EXACT && __any_sync(0xffffffffu, rmax > epi::R2_RECHECK))
+                    full = true;
             }
+#pragma unroll 1
+            for (int c = colh; full && c < it.bn() / CW; c += EPI_WARPS / 4) {   // the tile's chunks
+                uint32_t v[CW];
+                __syncwarp();
+                tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
+                if constexpr (MODE == R2_EXACT) {
+                    epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
+                                       c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
+                                       J.ldr, J.counts, J.ldc, 0, J.S);
+                    if (J.summary)
+                        acc.fold(v, it.b_row + c * CW, a, a_ok, J.n, J.symmetric,
+                                 J.threshold);
+                } else {
+                    // the F32 accumulators hold the counts as floats
+                    epi::chunk_ref<0, true, CW>(v, ra, colsr, c * CW, it.b_row + c * CW, a,
+                                                a_ok, n_tile, dlo, dhi, J.r2, J.ldr,
+                                                J.counts, J.ldc, 0, J.S);
+                }
+            }
+            tc_fence_before();
             __syncwarp();
-            if (lane == 0) release_item(qi);
-            named_bar_sync(1, R::EPI_THREADS);   // column factors may be rewritten
+            if (lane == 0) {
+                mbar_arrive_rank(smem_u32(&accempty[ab]), 0);
+                mbar_arrive(smem_u32(&facempty[ab]));
+                release_item(qi);
+            }
+            if (MODE == R2_EXACT && J.summary) acc.flush(J.summary);
+            __syncwarp();
         }
     }
 
@@ -557,7 +578,7 @@ cudaError_t launch_mode(const BatchParams &bp, int max_ctas, cudaStream_t st) {
             return e;
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = dim3(2 * (sms / 2), 1, 1);
-        cfg.blockDim = dim3(Roles<MODE>::THREADS, 1, 1);
+        cfg.blockDim = dim3(THREADS, 1, 1);
         cfg.dynamicSmemBytes = Smem<MODE>::BYTES;
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess || n <= 0) {
@@ -569,7 +590,7 @@ cudaError_t launch_mode(const BatchParams &bp, int max_ctas, cudaStream_t st) {
     long long pairs = bp.nitems < g_max_pairs ? bp.nitems : g_max_pairs;
     if (max_ctas > 0 && 2 * pairs > max_ctas) pairs = max_ctas / 2;
     if (pairs <= 0) return cudaSuccess;
-    kern<<<(int)(2 * pairs), Roles<MODE>::THREADS, Smem<MODE>::BYTES, st>>>(bp);
+    kern<<<(int)(2 * pairs), THREADS, Smem<MODE>::BYTES, st>>>(bp);
     return cudaGetLastError();
 }
 
