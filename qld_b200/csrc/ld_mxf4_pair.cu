@@ -70,6 +70,7 @@ constexpr int BM = RowTiles::BM, BN = 240;        // output tile of a pair
 constexpr int HM = 128, HN = 120;        // A and B rows held by each CTA
 constexpr int PW = 8;                    // packed words per row per packed stage
 constexpr int SUB = 2;                   // unpacked stages (256 samples) per packed stage
+constexpr int SW = PW / SUB;             // words per row per unpacked stage
 constexpr int UST = 4;                   // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;    // 8 KB
 constexpr int P_MAX = (HM + HN) * PW * 8;   // up to 15.5 KB delivered per stage
@@ -111,7 +112,7 @@ struct Smem {
                   "swizzled stages must start on whole swizzle atoms");
     // a group sees every (GROUPS / 2)-th packed stage or so: a slot must
     // always belong to the same groups for its phase bit to be enough
-    static_assert(PST * SUB % GROUPS == 0 && GROUPS <= UST, "stage rings");
+    static_assert(PST * SUB % GROUPS == 0 && GROUPS == UST && GROUPS % SUB == 0, "stage rings");
 };
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
 static_assert(SUB == 2 && EPI_WARPS * 32 == COLS_N && EPI_WARPS == 8, "work split");
@@ -159,6 +160,13 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int warp = tid >> 5, lane = tid & 31;
     const int np = (p.K + PW - 1) / PW;
     const int nu = np * SUB;
+    // Stages that hold samples: a tile's last one is all padding if K mod 8 is 1
+    // to 4, and is neither unpacked nor multiplied (29,817 SNPs, K = 260: 1,986 ->
+    // 1,975 us; 9,001 x 7,003 in reference mode with counts 336 -> 333).  Tiles of
+    // up to six stages keep it: they wait for their results' stores, which take
+    // turns of their own (9,001 x 7,003, K = 18: 77 -> 83 us without it, but
+    // 9,000 x 7,000 75 -> 73).
+    const int nu_k = np > 3 ? (p.K + SW - 1) / SW : nu;
 
     if (tid == 0) {
         for (int s = 0; s < PST; ++s) {
@@ -261,11 +269,13 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     tc_fence_after();
                     const uint32_t da = a_lo + s * (U_BYTES >> 4), db = da + (UA_BYTES >> 4);
                     if (elect_one()) {
+                        if (u < nu_k) {
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
-                                                (kk & 1) ? odd : even,
-                                                (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                            for (int kk = 0; kk < 4; ++kk)
+                                tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
+                                                    (kk & 1) ? odd : even,
+                                                    (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                        }
                         tc_commit_pair(smem_u32(&uempty[s]), BOTH);
                     }
                     __syncwarp();
@@ -279,35 +289,38 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     } else if (warp < FIRST_EPI_WARP) {
         // --------------------------------------------------------- unpack --
-        // group g takes the unpacked stages gu = g, g + GROUPS, ...
+        // Group g takes the unpacked stages gu = g, g + GROUPS, ...: always buffer
+        // g and the same half of every other packed slot, so slot and phases
+        // are counted up rather than divided out of gu and one vote serves
+        // both waits (9,001 x 7,003 in reference mode with counts 340 -> 336 us,
+        // 3,300 SNPs at K = 200 34.5 -> 33.1, single region 1,991 -> 1,986).
         const int grp = (warp - FIRST_UNPACK_WARP) / GROUP_WARPS;
         const mxf4rows::RowLane<GROUP_THREADS> rows(
             ((warp - FIRST_UNPACK_WARP) % GROUP_WARPS) * 32 + lane);
         const int total_u = my_tiles * nu;
+        uint8_t *const dst = smem + L::OFF_U + grp * U_BYTES;
+        const uint32_t uf = smem_u32(&ufull[grp]), ue = smem_u32(&uempty[grp]);
+        int ps = grp / SUB, u = grp % nu;    // packed slot; the stage's place in its tile
+        uint32_t ph = 0, eh = 1;             // phases of the packed slot and of the unpacked stage
         for (int gu = grp; gu < total_u; gu += GROUPS) {
-            const int gp = gu / SUB;
-            const int ps = gp % PST;
-            const bool got = mbar_wait(smem_u32(&pfull[ps]), (gp / PST) & 1, p.timeout_cycles,
-                                       p.status);
-            if (!__all_sync(0xffffffffu, got)) {
-                if (lane == 0) flag_error(p.status, ST_TIMEOUT_FULL);
-                break;
-            }
-            const int us = gu % UST;
-            const bool freed = gu < UST || mbar_wait(smem_u32(&uempty[us]), ((gu / UST) - 1) & 1,
-                                                     p.timeout_cycles, p.status);
+            const bool got = mbar_wait(smem_u32(&pfull[ps]), ph, p.timeout_cycles, p.status);
+            const bool freed = got && (gu < UST || mbar_wait(ue, eh, p.timeout_cycles, p.status));
             if (!__all_sync(0xffffffffu, freed)) {
-                if (lane == 0) flag_error(p.status, ST_TIMEOUT_MMA);
+                if (lane == 0) flag_error(p.status, got ? ST_TIMEOUT_MMA : ST_TIMEOUT_FULL);
                 break;
             }
-            mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(rows, HM + hn, smem + L::OFF_P + ps * P_BYTES,
-                                                        smem + L::OFF_U + us * U_BYTES, gu & 1);
+            if (u < nu_k)
+                mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(
+                    rows, HM + hn, smem + L::OFF_P + ps * P_BYTES, dst, grp % SUB);
             fence_proxy_async_smem();
             __syncwarp();
             if (lane == 0) {
-                mbar_arrive_rank(smem_u32(&ufull[us]), 0);
+                mbar_arrive_rank(uf, 0);
                 mbar_arrive(smem_u32(&pempty[ps]));     // one group per sub-stage
             }
+            eh ^= 1;
+            for (u += GROUPS; u >= nu;) u -= nu;
+            if ((ps += GROUPS / SUB) >= PST) ps -= PST, ph ^= 1;
         }
     } else if (FW && warp == FACTOR_WARP) {
         // ------------------------------------------------- column factors --
