@@ -56,6 +56,7 @@ constexpr int BM = RowTiles::BM, BN = 240;  // work item: output tile of a pair 
 constexpr int HM = 128, HN = 120;           // A and B rows held by each CTA
 constexpr int PW = 8;                       // packed words per row per packed stage
 constexpr int SUB = 2;                      // unpacked stages (256 samples) per packed stage
+constexpr int SW = PW / SUB;                // words per row per unpacked stage
 constexpr int UST = 4;                      // one unpacked stage per unpack group
 constexpr int PA_BYTES = HM * PW * 8;       // 8 KB
 constexpr int P_MAX = (HM + HN) * PW * 8;   // up to 15.5 KB delivered per stage
@@ -105,16 +106,21 @@ struct Smem {
                   "swizzled stages must start on whole swizzle atoms");
     // group g takes sub-stage g % 2 of packed stages g / 2, g / 2 + 2, ...: a
     // slot always belongs to the same two groups
-    static_assert(PST % 2 == 0 && GROUPS == 2 * SUB && GROUPS <= UST, "stage rings");
+    static_assert(PST % 2 == 0 && GROUPS == 2 * SUB && GROUPS == UST, "stage rings");
 };
 static_assert(ACC_STRIDE + BN <= SF_COL && SF_COL + 16 <= TMEM_COLS, "TMEM map");
 static_assert(SUB == 2 && EPI_WARPS % 4 == 0, "work split");
 
 // A work item: task (< 0: end of the queue), its tile's first A and B row, and
-// the packed stages (low 24 bits) and tile rows / 16 (high 8) of the task.
+// the words per row (low 24 bits) and tile rows / 16 (high 8) of the task.
 struct Item {
     int job, a_row, b_row, shape;
-    __device__ __forceinline__ int np() const { return shape & 0xFFFFFF; }
+    __device__ __forceinline__ int words() const { return shape & 0xFFFFFF; }
+    __device__ __forceinline__ int np() const { return (words() + PW - 1) / PW; }
+    // stages that hold samples, as ld_mxf4_pair.cu's nu_k
+    __device__ __forceinline__ int nu_k() const {
+        return np() > 3 ? (words() + SW - 1) / SW : np() * SUB;
+    }
     __device__ __forceinline__ int bn() const { return (shape >> 24) * 16; }
 };
 static_assert(sizeof(Item) == 16, "an item is one 16-byte record");
@@ -138,7 +144,7 @@ __device__ __forceinline__ Item decode_item(const BatchJob *jobs, int njobs, lon
     it.job = lo;
     int t = 0, base = 0;
     tl.decode_from((int)(g - J.item0), it.a_row, it.b_row, t, base);
-    it.shape = (J.K + PW - 1) / PW | (J.bn / 16) << 24;
+    it.shape = J.K | (J.bn / 16) << 24;
     return it;
 }
 
@@ -317,7 +323,7 @@ k_ld_batch(const BatchParams bp) {
                 if (it.job < 0) break;
                 const uint32_t even = idesc_mxf4_sf(BM, it.bn(), 0);   // k-steps 0, 2: scale bytes 0-1
                 const uint32_t odd = idesc_mxf4_sf(BM, it.bn(), 2);    // k-steps 1, 3: scale bytes 2-3
-                const int nu = it.np() * SUB;
+                const int nu = it.np() * SUB, nu_k = it.nu_k();
                 const int ab = it_n & 1;
                 if (it_n >= 2) {
                     const bool free = mbar_wait(smem_u32(&accempty[ab]), ((it_n >> 1) - 1) & 1,
@@ -339,11 +345,13 @@ k_ld_batch(const BatchParams bp) {
                     tc_fence_after();
                     const uint32_t da = a_lo + s * (U_BYTES >> 4), db = da + (UA_BYTES >> 4);
                     if (elect_one()) {
+                        if (u < nu_k) {
 #pragma unroll
-                        for (int kk = 0; kk < 4; ++kk)
-                            tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
-                                                (kk & 1) ? odd : even,
-                                                (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                            for (int kk = 0; kk < 4; ++kk)
+                                tc_mma_mxf4_pair_lo(d, da + kk * 2, db + kk * 2,
+                                                    (kk & 1) ? odd : even,
+                                                    (u > 0 || kk > 0) ? 1u : 0u, sf, sf);
+                        }
                         tc_commit_pair(smem_u32(&uempty[s]), BOTH);
                     }
                     __syncwarp();
@@ -363,8 +371,13 @@ k_ld_batch(const BatchParams bp) {
         const int grp = (warp - FIRST_UNPACK_WARP) / GROUP_WARPS;
         const mxf4rows::RowLane<GROUP_THREADS> rows(
             ((warp - FIRST_UNPACK_WARP) % GROUP_WARPS) * 32 + lane);
-        int gp = 0;
-        bool ok = true;
+        // slot and phases counted up, as in ld_mxf4_pair.cu: the group's stages are
+        // buffer grp and the same half of every other packed slot
+        uint8_t *const dst = smem + L::OFF_U + grp * U_BYTES;
+        const uint32_t uf = smem_u32(&ufull[grp]), ue = smem_u32(&uempty[grp]);
+        int ps = grp / SUB, kp = grp / SUB;  // packed slot; the stage's place in the item
+        uint32_t ph = 0, eh = 1;             // phases of the packed slot and of the unpacked stage
+        bool ok = true, first = true;
         for (int qi = 0; ok; ++qi) {
             const bool got_item = wait_item(qi);
             if (!__all_sync(0xffffffffu, got_item)) {
@@ -373,35 +386,29 @@ k_ld_batch(const BatchParams bp) {
             }
             const Item it = items[qi % QSLOTS];
             if (it.job < 0) break;
-            const int np = it.np(), nrows = HM + it.bn() / 2;
-            for (int kp = 0; kp < np; ++kp, ++gp) {
-                if ((gp & 1) != grp / SUB) continue;
-                const int ps = gp % PST;
-                const bool got = mbar_wait(smem_u32(&pfull[ps]), (gp / PST) & 1, limit, bp.status);
-                if (!__all_sync(0xffffffffu, got)) {
-                    if (lane == 0) flag_error(bp.status, ST_TIMEOUT_FULL);
-                    ok = false;
-                    break;
-                }
-                const int gu = gp * SUB + grp % SUB;
-                const int us = gu % UST;
-                const bool freed = gu < UST || mbar_wait(smem_u32(&uempty[us]),
-                                                         ((gu / UST) - 1) & 1, limit, bp.status);
+            const int np = it.np(), nu_k = it.nu_k(), nrows = HM + it.bn() / 2;
+            for (; kp < np; kp += GROUPS / SUB) {
+                const bool got = mbar_wait(smem_u32(&pfull[ps]), ph, limit, bp.status);
+                const bool freed = got && (first || mbar_wait(ue, eh, limit, bp.status));
                 if (!__all_sync(0xffffffffu, freed)) {
-                    if (lane == 0) flag_error(bp.status, ST_TIMEOUT_MMA);
+                    if (lane == 0) flag_error(bp.status, got ? ST_TIMEOUT_MMA : ST_TIMEOUT_FULL);
                     ok = false;
                     break;
                 }
-                mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(
-                    rows, nrows, smem + L::OFF_P + ps * P_BYTES, smem + L::OFF_U + us * U_BYTES,
-                    grp % SUB);
+                if (kp * SUB + grp % SUB < nu_k)
+                    mxf4rows::unpack_rows<GROUP_THREADS, TASKS>(
+                        rows, nrows, smem + L::OFF_P + ps * P_BYTES, dst, grp % SUB);
                 fence_proxy_async_smem();
                 __syncwarp();
                 if (lane == 0) {
-                    mbar_arrive_rank(smem_u32(&ufull[us]), 0);
+                    mbar_arrive_rank(uf, 0);
                     mbar_arrive(smem_u32(&pempty[ps]));
                 }
+                first = false;
+                eh ^= 1;
+                if ((ps += GROUPS / SUB) >= PST) ps -= PST, ph ^= 1;
             }
+            kp -= np;                        // its first stage of the next item
             __syncwarp();
             if (lane == 0) release_item(qi);
         }
