@@ -1192,7 +1192,7 @@ int qld_cuda_vcf_pack(qld_ctx *c, const char *text, size_t text_bytes,
     const int scratch_cap = K * 64;
     const size_t ns = (size_t)nsites;
     int rc;
-    if ((rc = ensure(c, c->vText, (text_bytes + 16) / 16 * 16)) ||
+    if ((rc = ensure(c, c->vText, text_bytes ? text_bytes : 1)) ||
         (rc = ensure(c, c->vSites, ns * sizeof(qld_vcf_site))) ||
         (rc = ensure(c, c->vValid, (size_t)nsamples)) || (rc = ensure(c, c->vSlash, ns * 8)) ||
         (rc = ensure(c, c->vRoff, ns * 8)) ||

@@ -251,14 +251,19 @@ k_vcf_sites(const char *__restrict__ text, const qld_vcf_site *__restrict__ site
         const char *t = text + site.off;
         uint32_t states = 0;             // site.states as one register
         for (int i = 0; i < 4; ++i) states |= (uint32_t)(uint8_t)site.states[i] << (8 * i);
-        // The line into shared memory, whole 16-byte words (the text buffer is
-        // padded to one): every thread then walks its own byte chunk, whose
-        // byte loads would each touch a dozen lines of global memory per warp.
+        // The line into shared memory, in 16-byte words up to its last few
+        // bytes: every thread then walks its own byte chunk, whose byte loads
+        // would each touch a dozen lines of global memory per warp.
         const int shift = (int)(site.off & 15);
         const bool staged = shift + len <= stage_bytes;
         if (staged) {
             const uint4 *src = reinterpret_cast<const uint4 *>(t - shift);
-            for (int i = threadIdx.x; i < (shift + len + 15) / 16; i += THREADS) stage[i] = src[i];
+            const int whole = (shift + len) >> 4, rest = (shift + len) & 15;
+            char last = 0;
+            if ((int)threadIdx.x < rest)
+                last = reinterpret_cast<const char *>(src + whole)[threadIdx.x];
+            for (int i = threadIdx.x; i < whole; i += THREADS) stage[i] = src[i];
+            if ((int)threadIdx.x < rest) reinterpret_cast<char *>(stage + whole)[threadIdx.x] = last;
             t = reinterpret_cast<const char *>(stage) + shift;
         }
         __syncthreads();
