@@ -272,7 +272,8 @@ def smem_roofline(m, n, K, symmetric, kern_ms, sm_mhz, sms=148):
     256-sample stage its 248 rows (128 A + 120 B) each take 32 B of TMA
     writes (packed words), 32 B of unpack reads, 128 B of E2M1 stores and
     128 B of tensor-core operand reads -- 320 B per row, the minimum of this
-    layout -- over two CTAs per tile and 2 * ceil(K / 8) stages per tile;
+    layout -- over two CTAs per tile and 2 * ceil(K / 8) stages per tile (the
+    kernel leaves out a last one of padding only, K mod 8 in 1..4);
     against 128 B per clock per SM at the sampled SM clock (nominal)."""
     if not kern_ms or not sm_mhz:
         return None

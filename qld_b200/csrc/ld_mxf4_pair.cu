@@ -31,8 +31,8 @@
 //                proxy fence, arrive: ~1,250 cycles by clock64), so two groups
 //                (of five warps) handed a stage over only every ~650 cycles,
 //                whatever the tensor cores and shared memory allowed; with
-//                four a stage takes ~600, at the shared-memory bound (620
-//                wavefronts).  Single region 2.36 -> 2.12 ms (first 100
+//                four a stage takes ~580, where the MMAs alone take 523 (565 at
+//                the rate they keep up back to back).  Single region 2.36 -> 2.12 ms (first 100
 //                launches; 2.41 -> 2.21 in a power-capped loop), 5,000-wide
 //                band 3.26 -> 2.80 ms, 9,001 x 7,003 x 16,622 reference mode
 //                with counts 403 -> 349 us.  Three groups of three: 2.16 ms /
