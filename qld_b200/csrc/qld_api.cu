@@ -17,9 +17,14 @@
 #include <utility>
 #include <vector>
 
+#include "launch_util.h"
 #include "qld_cuda.h"
 #include "qld_kernels.h"
 #include "tcgen05.cuh"
+
+namespace qld {
+std::atomic<unsigned> g_context_epoch{0};
+}
 
 using namespace qld;
 
@@ -764,6 +769,7 @@ int qld_cuda_init(int device, qld_ctx **ctx_out) {
     c->sm_count = prop.multiProcessorCount;
     if (const char *s = getenv("QLD_TIMEOUT_CYCLES")) c->timeout_cycles = atoll(s);
     int rc = QLD_OK;
+    g_context_epoch.fetch_add(1, std::memory_order_acq_rel);
     do {
         if (cudaSetDevice(device) != cudaSuccess) { rc = QLD_ERR_CUDA; break; }
         if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||
