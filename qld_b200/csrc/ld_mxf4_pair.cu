@@ -352,7 +352,8 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     special |= epi::store_col_ref(epi::ColsR2(base, COLS_N), i * 32 + lane, cb[i],
                                                   p.S);
             }
-            special = __any_sync(0xffffffffu, special);   // and every lane's factors are stored
+            special = __any_sync(0xffffffffu, special);
+            __syncwarp();                // every lane's factors are stored: a vote does not order them
             if (lane == 0) {
                 col_flag[ab] = special;
                 mbar_arrive(smem_u32(&facfull[ab]));
