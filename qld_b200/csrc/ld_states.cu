@@ -35,11 +35,16 @@
 // settles every pair.  The results are the same for any input, and rows that
 // defeat every shortcut cost one walk over all their words.
 //
-// Bound by integer issue: ~19 instructions per pair and word, 9.8 us per word
-// of a 4,001-SNP single region, over 4 words instead of K.  4,001 SNPs x
-// 16,622 samples (K = 260) of founder haplotypes with 1 % noise: 2,367 us with
-// one POPC per pair and word over all words, 64 now; one bit per row: 211;
-// dense random rows: 52; rows built to defeat every shortcut (all ones): 2,540.
+// Bound by integer issue: 13 instructions per pair and word (two LOP3 per joint
+// state, the second setting the predicate of an addition, and a permutation),
+// 6.8-8.0 us per word of a 4,001-SNP single region, over 4 words instead of K.
+// With compares and selects between them, 19 instructions, tables of up to
+// seven words and rows that defeat every shortcut took longer than the forward
+// fold (one POPC per pair and word, over all words).  In us, forward fold / 19
+// instructions / 13: 200 SNPs x 300 samples (K = 5) 17.3 / 19.0 / 15.3; 64 SNPs
+// of K = 2 8.1 / 10.5 / 8.0; 4,001 SNPs x 16,622 samples (K = 260) all ones
+// 2,368 / 2,531 / 2,089, 24 founder haplotypes with 1 % noise 2,365 / 61 / 54, one
+// bit per row 2,367 / 209 / 202, dense random rows 2,367 / 49 / 42.
 //
 // One CTA per 128 x 128 tile, 256 threads: lane l holds A rows l + 32 i, warp
 // w B rows 16 w + j, a thread 4 x 16 pairs, so a store writes 32 consecutive
@@ -62,19 +67,32 @@ constexpr int LIST_WORDS = 64;           // words each of them may take
 constexpr uint32_t START = 0x04030201u;  // F before any word
 
 // F o f_S for one word pair (32-bit halves).  Byte i of the result is byte
-// f_S(i + 1) - 1 of F, and f_S(v) = popc(v | S) = popc(S) + popc(v & ~S): as a
-// permutation selector, state 00 adds 1 to every nibble if present and to
-// those of v = 1 and 3 if not, 01 likewise v = 2 and 3, 10 v = 4, 11 none.
-// `entry` is all ones, or zero for word 0, whose v = 0 has no bit to add.
-__device__ __forceinline__ uint32_t before(uint32_t F, uint2 a, uint2 b, uint32_t entry) {
-    const uint32_t s11 = (a.x & b.x) | (a.y & b.y);
-    const uint32_t s10 = (a.x & ~b.x) | (a.y & ~b.y);
-    const uint32_t s01 = (~a.x & b.x) | (~a.y & b.y);
-    const uint32_t s00 = ~((a.x | b.x) & (a.y | b.y));
-    const uint32_t sel = (s00 != 0u ? 0x1111u : 0x0101u & entry) +
-                         (s01 != 0u ? 0x1111u : 0x0110u & entry) +
-                         (s10 != 0u ? 0x1111u : 0x1000u & entry) +
-                         (s11 != 0u ? 0u : 0u - 0x1111u);
+// f_S(i + 1) - 1 of F, and f_S(v) = popc(v | S): as a permutation selector, a
+// nibble for each v = 1..4, state 00 adds 1 to those of v = 2 and 4 if present,
+// 01 to v = 1 and 4, 10 to v = 1, 2 and 3, 11 to all, and v = 3 starts from 1.
+// Before word 0 st is 0: every state adds 1 to every nibble, and they start
+// from -1.
+struct Terms {
+    uint32_t base, c00, c01, c10;
+    __device__ __forceinline__ explicit Terms(bool word0)
+        : base(word0 ? 0u - 0x1111u : 0x0100u), c00(word0 ? 0x1111u : 0x1010u),
+          c01(word0 ? 0x1111u : 0x1001u), c10(word0 ? 0x1111u : 0x0111u) {}
+};
+// x += c if LUT(t, u, v) has a bit: the LOP3's own predicate, without a compare.
+template <int LUT>
+__device__ __forceinline__ void add_if(uint32_t &x, uint32_t t, uint32_t u, uint32_t v, uint32_t c) {
+    asm("{\n\t.reg .pred p, f;\n\t.reg .b32 d;\n\t"
+        "setp.ne.u32 f, 0, 0;\n\t"
+        "lop3.or.b32 d|p, %1, %2, %3, %5, f;\n\t"
+        "@p add.u32 %0, %0, %4;\n\t}"
+        : "+r"(x) : "r"(t), "r"(u), "r"(v), "r"(c), "n"(LUT));
+}
+__device__ __forceinline__ uint32_t before(uint32_t F, uint2 a, uint2 b, const Terms &t) {
+    uint32_t sel = t.base;
+    add_if<0xF8>(sel, a.x & b.x, a.y, b.y, 0x1111u);
+    add_if<0xF4>(sel, a.x & ~b.x, a.y, b.y, t.c10);
+    add_if<0xF2>(sel, ~a.x & b.x, a.y, b.y, t.c01);
+    add_if<0x1F>(sel, a.x | b.x, a.y, b.y, t.c00);
     return __byte_perm(F, F, sel);
 }
 
@@ -104,7 +122,7 @@ __device__ __noinline__ uint32_t walk_back(const uint64_t *a, const uint64_t *b,
             }
 #pragma unroll
         for (int q = 0; q < 8; ++q)
-            if (k0 - 1 - q >= stop) F = before(F, wa[q], wb[q], k0 - 1 - q == 0 ? 0u : ~0u);
+            if (k0 - 1 - q >= stop) F = before(F, wa[q], wb[q], Terms(k0 - 1 - q == 0));
         const uint32_t v = settled(F);
         if (v) return v;
     }
@@ -140,16 +158,18 @@ __global__ void __launch_bounds__(THREADS, 2) k_states(const StatesParams p) {
         is_a ? p.A + (long long)row * p.lda : p.B + (long long)row * p.ldb;
     uint2 *row_smem = is_a ? &sA[0][tid] : &sB[0][tid - BM];
 
-    // pairs the task does not have count as finished
-    uint64_t done = 0;
+    // pairs the task does not have count as finished (0.5 us of a small table's
+    // time when asked pair by pair)
+    static_assert(NI == 4 && NI * NJ == 64, "a bit per pair");
+    uint64_t done = ~0ull;
 #pragma unroll
-    for (int j = 0; j < NJ; ++j)
-#pragma unroll
-        for (int i = 0; i < NI; ++i) {
-            const int a = my_a + 32 * i, b = my_b + j;
-            const bool need = a < p.m && b < p.n && (!p.symmetric || a >= b);
-            done |= (uint64_t)(!need) << (j * NI + i);
-        }
+    for (int i = 0; i < NI; ++i) {
+        const int a = my_a + 32 * i;
+        int n = (p.symmetric && a + 1 < p.n ? a + 1 : p.n) - my_b;   // my first n B rows count
+        n = a < p.m && n > 0 ? (n < NJ ? n : NJ) : 0;
+        const uint64_t mine = n == NJ ? ~0ull : (1ull << (NI * n)) - 1ull;
+        done &= ~(mine & 0x1111111111111111ull << i);
+    }
     auto put = [&](int j, int i, uint32_t st) {
         p.out[(long long)(my_b + j - p.out_row0) * p.lds + my_a + 32 * i] = (uint8_t)st;
         done |= 1ull << (j * NI + i);
@@ -162,7 +182,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_states(const StatesParams p) {
         for (int i = 0; i < NI; ++i) x[j][i] = START;
 
     // up to SHORT words at once: what follows the first four costs more than one
-    // word does (200 SNPs x 300 samples 22.8 -> 20.7 us; at K = 8 24.8 -> 28.9)
+    // word does (200 SNPs x 300 samples 17.4 -> 15.3 us; all of K = 8 17.4 -> 21.2)
     long long len = p.K <= SHORT ? p.K : W;
     for (int end = p.K;; len *= 4) {
         const int s0 = end > len ? (int)(end - len) : 0;
@@ -178,7 +198,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_states(const StatesParams p) {
             const int words = e - s0 < W ? e - s0 : W;
 #pragma unroll 1
             for (int w = 0; w < words; ++w) {
-                const uint32_t entry = e - 1 - w == 0 ? 0u : ~0u;
+                const Terms terms(e - 1 - w == 0);
                 uint2 a[NI];
 #pragma unroll
                 for (int i = 0; i < NI; ++i) a[i] = sA[w][lane + 32 * i];
@@ -186,7 +206,7 @@ __global__ void __launch_bounds__(THREADS, 2) k_states(const StatesParams p) {
                 for (int j = 0; j < NJ; ++j) {
                     const uint2 b = sB[w][warp * NJ + j];
 #pragma unroll
-                    for (int i = 0; i < NI; ++i) x[j][i] = before(x[j][i], a[i], b, entry);
+                    for (int i = 0; i < NI; ++i) x[j][i] = before(x[j][i], a[i], b, terms);
                 }
             }
         }
