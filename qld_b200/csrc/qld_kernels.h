@@ -116,8 +116,7 @@ cudaError_t launch_states(const StatesParams &p, int tiles_b, cudaStream_t st);
 // the random draws the others need (slash_count) with their row length and
 // errors; the second packs those, drawing site s's numbers from
 // rnd[rnd_off[s]...].  Each CTA uses scratch_cap bytes of scratch (>= K * 64).
-// text is readable up to the next multiple of 16 bytes past its end; max_len
-// bounds the sites' len.
+// max_len bounds the sites' len; nothing past a line's last byte is read.
 enum VcfError {
     QLD_VCF_OK = 0,
     QLD_VCF_EMPTY_GT = 1,     // the GT subfield is empty
