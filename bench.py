@@ -350,6 +350,13 @@ def _blis_threads(jc, ic):
     os.environ["OMP_NUM_THREADS"] = str(jc * ic)
 
 
+def reference_unavailable():
+    """Why the reference's CPU path cannot run here, or None."""
+    if _oracle().ref_available():
+        return None
+    return "the reference library is not built here (oracle/_ref needs the qLD sources)"
+
+
 def cpu_reference_sample(T_np, S, ms, factoring=None):
     """One timed run of the reference's stock -blis path on the first `ms`
     SNPs of the table (single region): BLIS cblas_dsyrk counts (BLIS threads
@@ -446,7 +453,11 @@ def cpu_reference_tasks(tasks):
 def cpu_sampled_baseline(make_tasks, sizes, seconds_target=6.0):
     """cpu_baseline of a section: make_tasks(size) -> (tasks, pairs, description)
     for a growing sample size; the first size is a probe whose time sets the
-    final size (time taken as proportional to size, capped at sizes[1])."""
+    final size (time taken as proportional to size, capped at sizes[1]).  Without
+    the reference library only the reason stands there."""
+    why = reference_unavailable()
+    if why:
+        return {"unavailable": why}
     model, phys, _ = host_cpu()
     probe, cap = sizes
     tasks, pairs, _ = make_tasks(probe)
@@ -488,6 +499,10 @@ def reference_arm(args, rank, world):
     import numpy as np
     cfg = arm_config(args, world)
     if rank != 0:
+        return
+    why = reference_unavailable()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return
     T, S = make_table(args.workload, "cpu")
     T_np = T.numpy().view(np.uint64)
@@ -753,7 +768,9 @@ def ours_arm(args, rank, world, local_rank):
                        "api": "qld_cuda_ld (pinned host buffers)"}
         del Th, bch, outh
 
-    if rank == 0 and world == 1 and not args.no_cpu:
+    if rank == 0 and world == 1 and not args.no_cpu and reference_unavailable():
+        line["cpu_baseline"] = {"unavailable": reference_unavailable()}
+    elif rank == 0 and world == 1 and not args.no_cpu:
         T_np = T.cpu().numpy().view(np.uint64)
         fac = best_blis_factoring(T_np, S)
         if fac:

@@ -283,6 +283,12 @@ def blis_available() -> bool:
     return os.path.exists(os.path.join(_HERE, "_ref", "libqldref_blis.so"))
 
 
+def ref_available() -> bool:
+    """Whether either form of the reference library was built here (they need the
+    qLD sources)."""
+    return blis_available() or os.path.exists(os.path.join(_HERE, "_ref", "libqldref.so"))
+
+
 def ref_blis_counts_ld(A, bc, S, B=None, bcB=None, C=None, results=None):
     """The reference's stock -blis path on one task (ref_blis.c): BLIS
     cblas_dsyrk (single region, lower triangle of C) or cblas_dgemm (two
