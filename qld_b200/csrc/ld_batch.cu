@@ -490,6 +490,8 @@ k_ld_batch(const BatchParams bp) {
                 tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)ab * ACC_STRIDE;
             const int n_tile = it.b_row + it.bn() < J.n ? it.b_row + it.bn() : J.n;
             const int dlo = diag_lo(J.symmetric, 0), dhi = diag_hi(0);
+            uint32_t *const counts = PLAIN ? nullptr : J.counts;
+            BatchSummary *const summary = PLAIN ? nullptr : J.summary;
             epi::SumAcc acc;
             // Chunks of 16 columns, in reference mode of 8 (more columns spill:
             // 32 in exact mode 620 us against 566 on 300 tasks, 16 in
@@ -529,15 +531,15 @@ k_ld_batch(const BatchParams bp) {
                 if constexpr (MODE == R2_EXACT) {
                     epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
                                        c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
-                                       J.ldr, J.counts, J.ldc, 0, J.S);
-                    if (J.summary)
+                                       J.ldr, counts, J.ldc, 0, J.S);
+                    if (summary)
                         acc.fold(v, it.b_row + c * CW, a, a_ok, J.n, J.symmetric,
                                  J.threshold);
                 } else {
                     // the F32 accumulators hold the counts as floats
                     epi::chunk_ref<0, true, CW>(v, ra, colsr, c * CW, it.b_row + c * CW, a,
                                                 a_ok, n_tile, dlo, dhi, J.r2, J.ldr,
-                                                J.counts, J.ldc, 0, J.S);
+                                                counts, J.ldc, 0, J.S);
                 }
             }
             tc_fence_before();
@@ -547,7 +549,7 @@ k_ld_batch(const BatchParams bp) {
                 mbar_arrive(smem_u32(&facempty[ab]));
                 release_item(qi);
             }
-            if (MODE == R2_EXACT && J.summary) acc.flush(J.summary);
+            if (MODE == R2_EXACT && summary) acc.flush(summary);
             __syncwarp();
         }
     }

@@ -127,7 +127,7 @@ static_assert(SUB == 2 && EPI_WARPS * 32 == COLS_N && EPI_WARPS == 8, "work spli
 // 50,000 x 10,001 199 -> 192, in reference mode 241 -> 222.  A branch in one
 // kernel cost the launches with counts 1 %.
 // FW: a warp of its own stores the column factors (otherwise the epilogue warps
-// do, after a tile's chunks; pair_factor_warp chooses).
+// do, after a tile's chunks; factor_warp chooses).
 template <int MODE, bool BAND, bool FULL, bool PLAIN, bool FW>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(threads(FW), 1)
 k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
@@ -618,13 +618,19 @@ int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
 // 265 -> 266, 327 -> 339; 12,000 SNPs, K = 80: 144 -> 132, 222 -> 187.
 // A launch of one or two waves gains less than the first tile's factors, all
 // from one warp, cost it: 3,300 SNPs, exact mode, K = 60 17.6 -> 17.8.
-bool factor_warp(const RowTiles &tl, int K, int r2_mode) {
+// Exact mode with counts writes twice the bytes, and warps that run apart write
+// the two parts of a 32-byte sector that rows of odd length share at distant times:
+// 11,734 x 10,140 SNPs, K = 3 346 us with the extra warp and 213 without (300
+// before either), at rows of whole sectors 167 and 183 (300); 8,547 x 4,813, K = 7
+// 116 and 87 (113); 9,001 x 7,003, K = 80 175 and 185 (218).
+bool factor_warp(const RowTiles &tl, int K, int r2_mode, bool counts) {
+    if (counts && r2_mode != R2_REFERENCE) return false;
     return K <= (r2_mode == R2_REFERENCE ? 160 : 100) && tl.count() > 2 * max_pairs();
 }
 
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              const RowTiles &tl, int r2_mode, cudaStream_t st) {
-    const bool fw = factor_warp(tl, p.K, r2_mode);
+    const bool fw = factor_warp(tl, p.K, r2_mode, p.counts != nullptr);
     if (r2_mode == R2_REFERENCE)
         return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
                    ? launch_rule<R2_REFERENCE, true>(fw, tmA, tmB, p, tl, st)
