@@ -591,7 +591,12 @@ __device__ __forceinline__ void chunk(uint32_t (&v)[32], const ARow &ra, const C
 // (c = 0), so that its pairs come out 0 without a test.  That fails only
 // against a factor that is not a finite, non-negative number -- a fixed SNP
 // (c = S: infinity) or a bit count above S -- which `special` reports: a warp
-// that holds or meets one applies the zero rule explicitly.
+// that holds or meets one applies the zero rule explicitly.  Tables with fixed
+// SNPs do that in nearly every tile, so the rule stands in the loop over the
+// pairs; as a second pass that read the columns again it made them slower than
+// a test in every launch had been (11,734 x 10,140 SNPs of K = 3 with 5 % fixed
+// and 5 % empty SNPs: such a test 166 us, second pass 218, now 152; K = 80, 9,001 x
+// 7,003 147 / 168 / 131; 300-row tasks in a batch 16.4 / 18.5 / 14.4).
 struct FactorF {
     float c, inv;
     bool special;
@@ -639,16 +644,45 @@ __device__ __forceinline__ float pair_r2_f64(float c, float ca, float cb, int S)
     return __double2float_rn(r);
 }
 
+// The FP32 values of a chunk's counts, in pairs of columns; their maximum folded
+// into rmax.  ZERO: with the zero rule, a pair of an empty SNP is 0 whatever the
+// other's factor (hi = cA cB is 0 there only).
+template <int CW, bool ZERO>
+__device__ __forceinline__ void chunk_values_f32(uint32_t (&v)[CW], const ARowF &ra,
+                                                 const ColsF &f, int bl0, float S_f, float &rmax) {
+    const f2 S2 = splat2(S_f), ca = splat2(ra.c), nca = splat2(-ra.c), ia = splat2(ra.inv);
+#pragma unroll
+    for (int t = 0; t < CW; t += 2) {
+        const ulonglong2 col = f.pair(bl0 + t);
+        const f2 cnt = pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1]));
+        const f2 nhi = mul2(nca, col.x);                       // -hi
+        const f2 lo = fma2(ca, col.x, nhi);
+        const f2 D = sub2(fma2(S2, cnt, nhi), lo);
+        float r0, r1;
+        unpack2(mul2(mul2(D, D), mul2(ia, col.y)), r0, r1);
+        if constexpr (ZERO) {
+            float h0, h1;
+            unpack2(nhi, h0, h1);
+            r0 = h0 == 0.0f ? 0.0f : r0;
+            r1 = h1 == 0.0f ? 0.0f : r1;
+        }
+        rmax = max3(rmax, r0, r1);
+        v[t] = __float_as_uint(r0);
+        v[t + 1] = __float_as_uint(r1);
+    }
+}
+
 // One chunk of CW (<= 32) columns of F32 accumulators v[t] (count c as float bits), as
 // chunk<R2_EXACT, 0> with the FP32 evaluation above.  taddr is the TMEM
 // address the chunk was loaded from: the rare pairs whose FP32 value lies
 // above 1.00009 are re-evaluated in FP64 from their count, reloaded one
 // column at a time (warp-uniform loads, off the common path).
-// cols_special: a column of the tile is `special`.
+// cols_special: a column of the tile is `special`.  RARE: a caller that comes here
+// with rare cases only, which takes the loop with the zero rule always.
 // The counts go out as plain or predicated stores: with a test and a branch per
 // column the arithmetic waited for each (11,776 x 10,140 SNPs, K = 3 298 -> 183
 // us, 9,001 x 7,003 of K = 130 249 -> 204).
-template <int CW = 32>
+template <int CW = 32, bool RARE = false>
 __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, const ARowF &ra,
                                           const ColsF &f, bool cols_special, int bl0, int b0,
                                           int a, bool a_ok, int n, int dlo, int dhi, float *r2,
@@ -668,26 +702,11 @@ __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, con
                          (mask >> t) & 1u);
         }
     }
-    const f2 S2 = splat2((float)S), ca = splat2(ra.c), nca = splat2(-ra.c), ia = splat2(ra.inv);
     float rmax = 0.0f;
-#pragma unroll
-    for (int t = 0; t < CW; t += 2) {
-        const ulonglong2 col = f.pair(bl0 + t);
-        const f2 cnt = pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1]));
-        const f2 nhi = mul2(nca, col.x);                       // -hi
-        const f2 lo = fma2(ca, col.x, nhi);
-        const f2 D = sub2(fma2(S2, cnt, nhi), lo);
-        float r0, r1;
-        unpack2(mul2(mul2(D, D), mul2(ia, col.y)), r0, r1);
-        rmax = max3(rmax, r0, r1);
-        v[t] = __float_as_uint(r0);
-        v[t + 1] = __float_as_uint(r1);
-    }
-    if (__any_sync(0xffffffffu, ra.special) || cols_special) {
-#pragma unroll
-        for (int t = 0; t < CW; ++t)
-            if (ra.c == 0.0f || f.c(bl0 + t) == 0.0f) v[t] = 0u;
-    }
+    if (RARE || __any_sync(0xffffffffu, ra.special) || cols_special)
+        chunk_values_f32<CW, true>(v, ra, f, bl0, (float)S, rmax);
+    else
+        chunk_values_f32<CW, false>(v, ra, f, bl0, (float)S, rmax);
     if (__any_sync(0xffffffffu, rmax > 1.00009f)) {
 #pragma unroll
         for (int t = 0; t < CW; ++t) {
@@ -729,20 +748,7 @@ __device__ __forceinline__ void chunk_f32_plain(uint32_t (&v)[CW], const ARowF &
                                                 int bl0, int b0, int a, bool a_ok, int n, int dlo,
                                                 int dhi, float *o, long long ldr, float S_f,
                                                 float &rmax) {
-    const f2 S2 = splat2(S_f), ca = splat2(ra.c), nca = splat2(-ra.c), ia = splat2(ra.inv);
-#pragma unroll
-    for (int t = 0; t < CW; t += 2) {
-        const ulonglong2 col = f.pair(bl0 + t);
-        const f2 cnt = pack2(__uint_as_float(v[t]), __uint_as_float(v[t + 1]));
-        const f2 nhi = mul2(nca, col.x);                       // -hi
-        const f2 lo = fma2(ca, col.x, nhi);
-        const f2 D = sub2(fma2(S2, cnt, nhi), lo);
-        float r0, r1;
-        unpack2(mul2(mul2(D, D), mul2(ia, col.y)), r0, r1);
-        rmax = max3(rmax, r0, r1);
-        v[t] = __float_as_uint(r0);
-        v[t + 1] = __float_as_uint(r1);
-    }
+    chunk_values_f32<CW, false>(v, ra, f, bl0, S_f, rmax);
     if (!a_ok) return;
     const bool interior = (b0 + CW - 1 < n) && (a - (b0 + CW - 1) >= dlo) && (a - b0 <= dhi);
     if (interior) {

@@ -460,7 +460,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<CW>(v, tbase + (uint32_t)(c * CW), raf,
+                        epi::chunk_f32<CW, PLAIN>(v, tbase + (uint32_t)(c * CW), raf,
                                            epi::ColsF(base, COLS_N), cols_special, c * CW,
                                            b_tile + c * CW, a, a_ok, n_tile, dlo, dhi, p.r2, p.ldr,
                                            p.counts, p.ldc, p.out_row0, p.S);
