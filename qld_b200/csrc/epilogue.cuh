@@ -445,15 +445,19 @@ __device__ __forceinline__ void chunk_ref(uint32_t (&v)[CW], const ARowR &ra, co
                 }
             }
         }
-        if (__any_sync(0xffffffffu, redo != 0)) {
+        // one reduction for the flagged columns, not a vote for each (twelve 200-450-row
+        // tasks of K = 3 with 5 % fixed and 5 % empty SNPs 30.6 -> 28.7 us, 300 tasks
+        // 1,064 -> 1,050)
+        const uint32_t columns = __reduce_or_sync(0xffffffffu, redo);
+        if (columns != 0u) {
             RowRef rA;
             rA.c = ra.c;
             rA.v = ra.k.x;
             rA.one_minus = __dsub_rn(1.0, (double)ra.k.x);
 #pragma unroll
             for (int t = 0; t < CW; ++t) {
-                const bool rd = (redo >> t) & 1u;
-                if (__any_sync(0xffffffffu, rd) && rd) {
+                if (!((columns >> t) & 1u)) continue;
+                if ((redo >> t) & 1u) {
                     const float4 cb = f.col(bl0 + t);
                     RowRef rb;
                     rb.c = cb.x != 0.0f;        // only the zero rule reads it
