@@ -681,12 +681,14 @@ __device__ __forceinline__ void chunk_values_f32(uint32_t (&v)[CW], const ARowF 
 // address the chunk was loaded from: the rare pairs whose FP32 value lies
 // above 1.00009 are re-evaluated in FP64 from their count, reloaded one
 // column at a time (warp-uniform loads, off the common path).
-// cols_special: a column of the tile is `special`.  RARE: a caller that comes here
-// with rare cases only, which takes the loop with the zero rule always.
+// cols_special: a column of the tile is `special`.  ONE: the loop with the zero
+// rule for every warp, for callers whose time one loop less of code is worth more
+// than the rule (65 tasks with counts in a batch 52.5 -> 49.4 us, with fixed SNPs
+// 57.5 -> 51.7; the single-SM kernel is 2 % faster with both).
 // The counts go out as plain or predicated stores: with a test and a branch per
 // column the arithmetic waited for each (11,776 x 10,140 SNPs, K = 3 298 -> 183
 // us, 9,001 x 7,003 of K = 130 249 -> 204).
-template <int CW = 32, bool RARE = false>
+template <int CW = 32, bool ONE = false>
 __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, const ARowF &ra,
                                           const ColsF &f, bool cols_special, int bl0, int b0,
                                           int a, bool a_ok, int n, int dlo, int dhi, float *r2,
@@ -707,7 +709,7 @@ __device__ __forceinline__ void chunk_f32(uint32_t (&v)[CW], uint32_t taddr, con
         }
     }
     float rmax = 0.0f;
-    if (RARE || __any_sync(0xffffffffu, ra.special) || cols_special)
+    if (ONE || __any_sync(0xffffffffu, ra.special) || cols_special)
         chunk_values_f32<CW, true>(v, ra, f, bl0, (float)S, rmax);
     else
         chunk_values_f32<CW, false>(v, ra, f, bl0, (float)S, rmax);

@@ -529,7 +529,7 @@ k_ld_batch(const BatchParams bp) {
                 __syncwarp();
                 tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                 if constexpr (MODE == R2_EXACT) {
-                    epi::chunk_f32<CW, PLAIN>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
+                    epi::chunk_f32<CW, true>(v, tbase + (uint32_t)(c * CW), raf, colsf, cols_special,
                                        c * CW, it.b_row + c * CW, a, a_ok, n_tile, dlo, dhi, J.r2,
                                        J.ldr, counts, J.ldc, 0, J.S);
                     if (summary)

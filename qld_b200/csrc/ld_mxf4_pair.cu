@@ -460,7 +460,7 @@ k_ld_mxf4_pair(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     __syncwarp();
                     tc_ld_32x32b<CW>(tbase + (uint32_t)(c * CW), v);
                     if constexpr (MODE == R2_EXACT) {
-                        epi::chunk_f32<CW, PLAIN>(v, tbase + (uint32_t)(c * CW), raf,
+                        epi::chunk_f32<CW, true>(v, tbase + (uint32_t)(c * CW), raf,
                                            epi::ColsF(base, COLS_N), cols_special, c * CW,
                                            b_tile + c * CW, a, a_ok, n_tile, dlo, dhi, p.r2, p.ldr,
                                            p.counts, p.ldc, p.out_row0, p.S);
@@ -618,19 +618,26 @@ int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
 // 265 -> 266, 327 -> 339; 12,000 SNPs, K = 80: 144 -> 132, 222 -> 187.
 // A launch of one or two waves gains less than the first tile's factors, all
 // from one warp, cost it: 3,300 SNPs, exact mode, K = 60 17.6 -> 17.8.
-// Exact mode with counts writes twice the bytes, and warps that run apart write
-// the two parts of a 32-byte sector that rows of odd length share at distant times:
-// 11,734 x 10,140 SNPs, K = 3 346 us with the extra warp and 213 without (300
-// before either), at rows of whole sectors 167 and 183 (300); 8,547 x 4,813, K = 7
-// 116 and 87 (113); 9,001 x 7,003, K = 80 175 and 185 (218).
-bool factor_warp(const RowTiles &tl, int K, int r2_mode, bool counts) {
-    if (counts && r2_mode != R2_REFERENCE) return false;
+// Counts beside r^2, in rows that do not start on 32-byte sectors (`odd_rows`):
+// warps that run apart write the two parts of a sector at distant times, and a
+// launch bound by its stores pays for it.  Without / with the extra warp, exact
+// mode: 11,734 x 10,140 K = 3 214 / 359, K = 40 278 / 331, 8,547 x 4,813 K = 7 87 / 116,
+// 9,001 x 7,003 K = 80 185 / 175; reference mode: 10,501 SNPs K = 3 295 / 329,
+// K = 20 333 / 378, K = 80 389 / 345, 7,001 x 6,999 K = 20 159 / 156.  In whole sectors
+// the extra warp pays as without counts: 11,776 x 10,140 K = 3 183 / 167, 12,000 SNPs
+// K = 20 in reference mode 425 / 384.
+bool factor_warp(const RowTiles &tl, int K, int r2_mode, bool odd_rows) {
+    if (odd_rows && (r2_mode != R2_REFERENCE || K < 40)) return false;
     return K <= (r2_mode == R2_REFERENCE ? 160 : 100) && tl.count() > 2 * max_pairs();
 }
 
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              const RowTiles &tl, int r2_mode, cudaStream_t st) {
-    const bool fw = factor_warp(tl, p.K, r2_mode, p.counts != nullptr);
+    const bool odd_rows =
+        p.counts && ((p.ldr | p.ldc) % 8 != 0 ||
+                     ((reinterpret_cast<uintptr_t>(p.r2) | reinterpret_cast<uintptr_t>(p.counts)) &
+                      31) != 0);
+    const bool fw = factor_warp(tl, p.K, r2_mode, odd_rows);
     if (r2_mode == R2_REFERENCE)
         return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
                    ? launch_rule<R2_REFERENCE, true>(fw, tmA, tmB, p, tl, st)

@@ -346,7 +346,7 @@ k_ld_mxf4_split(const __grid_constant__ CUtensorMap tmA, const __grid_constant__
                     }
                 }
                 if constexpr (MODE == R2_EXACT)
-                    epi::chunk_f32<CW, PLAIN>(v, taddr, raf, colsf, cols_special, col, b_row + col, a,
+                    epi::chunk_f32<CW, true>(v, taddr, raf, colsf, cols_special, col, b_row + col, a,
                                        a_ok, n_tile, dlo, dhi, p.r2, p.ldr, p.counts, p.ldc,
                                        p.out_row0, p.S);
                 else
