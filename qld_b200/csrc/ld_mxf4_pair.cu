@@ -618,26 +618,33 @@ int pair_tile_rows(const RowTiles &tl, int K, int r2_mode) {
 // 265 -> 266, 327 -> 339; 12,000 SNPs, K = 80: 144 -> 132, 222 -> 187.
 // A launch of one or two waves gains less than the first tile's factors, all
 // from one warp, cost it: 3,300 SNPs, exact mode, K = 60 17.6 -> 17.8.
-// Counts beside r^2, in rows that do not start on 32-byte sectors (`odd_rows`):
-// warps that run apart write the two parts of a sector at distant times, and a
-// launch bound by its stores pays for it.  Without / with the extra warp, exact
-// mode: 11,734 x 10,140 K = 3 214 / 359, K = 40 278 / 331, 8,547 x 4,813 K = 7 87 / 116,
-// 9,001 x 7,003 K = 80 185 / 175; reference mode: 10,501 SNPs K = 3 295 / 329,
-// K = 20 333 / 378, K = 80 389 / 345, 7,001 x 6,999 K = 20 159 / 156.  In whole sectors
-// the extra warp pays as without counts: 11,776 x 10,140 K = 3 183 / 167, 12,000 SNPs
-// K = 20 in reference mode 425 / 384.
-bool factor_warp(const RowTiles &tl, int K, int r2_mode, bool odd_rows) {
-    if (odd_rows && (r2_mode != R2_REFERENCE || K < 40)) return false;
-    return K <= (r2_mode == R2_REFERENCE ? 160 : 100) && tl.count() > 2 * max_pairs();
+// In rows that do not start on 32-byte sectors (`odd_rows`) warps that run apart
+// write the two parts of a sector at distant times, and a launch bound by its
+// stores pays for it: with counts beside r^2, and without in exact mode where
+// the output is several times the L2.  Without / with the extra warp, counts,
+// exact mode: 11,734 x 10,140 K = 3 214 / 359, K = 40 278 / 331, 8,547 x 4,813 K = 7
+// 87 / 116, 9,001 x 7,003 K = 80 185 / 175; reference mode: 10,501 SNPs K = 3 295 /
+// 329, K = 20 333 / 378, K = 80 389 / 345, 7,001 x 6,999 K = 20 159 / 156; no counts,
+// exact mode: 29,817 SNPs K = 4 524 / 665, K = 20 560 / 606, K = 30 643 / 542, 20,001 x
+// 9,000 K = 4 211 / 246, 9,001 x 7,003 K = 8 80 / 73.  In whole sectors the extra warp
+// pays: counts, 11,776 x 10,140 K = 3 183 / 167, 12,000 SNPs K = 20 in reference mode
+// 425 / 384; no counts, 29,824 SNPs K = 4 468 / 400.
+bool factor_warp(const RowTiles &tl, const LdParams &p, int r2_mode) {
+    const bool exact = r2_mode != R2_REFERENCE;
+    auto odd = [](const void *base, long long ld) {
+        return ld % 8 != 0 || (reinterpret_cast<uintptr_t>(base) & 31) != 0;
+    };
+    const int tiles = tl.count(), most = max_pairs();
+    if (odd(p.r2, p.ldr) || (p.counts && odd(p.counts, p.ldc))) {
+        if (p.counts && (exact || p.K < 40)) return false;
+        if (!p.counts && exact && p.K < 24 && tiles > 30 * most) return false;
+    }
+    return p.K <= (exact ? 100 : 160) && tiles > 2 * most;
 }
 
 cudaError_t launch_mxf4_pair(const CUtensorMap &tmA, const CUtensorMap &tmB, const LdParams &p,
                              const RowTiles &tl, int r2_mode, cudaStream_t st) {
-    const bool odd_rows =
-        p.counts && ((p.ldr | p.ldc) % 8 != 0 ||
-                     ((reinterpret_cast<uintptr_t>(p.r2) | reinterpret_cast<uintptr_t>(p.counts)) &
-                      31) != 0);
-    const bool fw = factor_warp(tl, p.K, r2_mode, odd_rows);
+    const bool fw = factor_warp(tl, p, r2_mode);
     if (r2_mode == R2_REFERENCE)
         return !p.counts && p.S >= epi::R2_PLAIN_S && p.S <= (1 << 24)
                    ? launch_rule<R2_REFERENCE, true>(fw, tmA, tmB, p, tl, st)
