@@ -25,8 +25,8 @@
 // slot on rank 0's barrier when done with its item.  A ticket past the last
 // item pushes an end marker.  With the TMA thread claiming and decoding its
 // items itself (an atomic and a binary search, ~4 us) and 240-row tiles
-// throughout, 300 tasks of 64-2,048 SNPs took 567 us against 533 (reference
-// mode 647 / 614).
+// throughout, the 300 tasks took 567 us against 533 (reference mode 647 /
+// 614).
 //
 // Roles per CTA (640 threads): warp 0 TMA of the CTA's rows, warp 1 TMEM and
 // (rank 0) the MMAs, warps 2-9 unpack in four groups taking the 256-sample
@@ -37,9 +37,12 @@
 // rows pay in full, the 300 tasks took 488 us against 472 (reference mode, then
 // with twelve epilogue warps, 588 against 549).  TMEM: two accumulators
 // (columns 0 and 256), so a tile's epilogue overlaps the next tile's MMAs,
-// and the scale factors at columns 496-511.  Every wait is bounded and no
-// thread returns early: both CTAs meet at the cluster barriers at start and
-// end on every path.
+// and the scale factors at columns 496-511.  Every wait on an mbarrier is bounded
+// and no thread returns early: both CTAs meet at the cluster barriers, which have
+// no limit, at start and end on every path.
+// The times here and below are of 300 tasks of 64-2,048 SNPs, as a replayed plan,
+// with and without the one change on the kernel of that day; it takes 457 us now,
+// 540 in reference mode.
 #include "epilogue.cuh"
 #include "mxf4_rows.cuh"
 #include "mxf4_tiles.cuh"
@@ -86,7 +89,7 @@ constexpr int QSLOTS = 4;                                    // item ring depth
 constexpr int ITEM_USERS = 2 * (1 + UNPACK_WARPS + EPI_WARPS + 1) + 1;
 
 // Shared-memory layout per r^2 mode: R2_EXACT needs 8 bytes of column
-// factors per column (epi::ColsF), R2_REFERENCE 16 (epi::ColsR); both leave
+// factors per column (epi::ColsF), R2_REFERENCE 16 (epi::ColsR2); both leave
 // room for six packed stages (more TMA lookahead than five).
 template <int MODE>
 struct Smem {

@@ -25,11 +25,12 @@
 //   warps 2-17   workers: unpack (w -> four words of nibbles, nibble n of
 //                output word t = bit 4n + t of w, the same permutation of
 //                the samples for A and B), then the epilogue: warp w reads
-//                TMEM lane quarter w % 4 of one accumulator, 4 of its 8
-//                32-column chunks, and applies the r^2 epilogue
-//                (gemm_cpu.c:343-404) on the way out.
-// Every wait is bounded; on expiry the kernel records the cause in the
-// status word and returns.
+//                TMEM lane quarter w % 4 of one accumulator, half of its
+//                chunks, and applies the r^2 epilogue (gemm_cpu.c:343-404)
+//                on the way out.
+// Every wait on an mbarrier is bounded; on expiry the kernel records the cause
+// in the status word and returns.  The workers' named barriers have no limit:
+// every worker warp meets both once a tile, also after a failed wait.
 #include "epilogue.cuh"
 #include "qld_kernels.h"
 #include "tcgen05.cuh"

@@ -50,9 +50,11 @@
 //                warps then neither divide for columns nor meet at a barrier,
 //                and each runs ahead of the others by up to a tile.  Where it
 //                pays: factor_warp() below.
-// Every wait is bounded.  No thread returns early: both CTAs meet at the
-// cluster barriers at start and end on every path, including after a
-// timeout, and the TMEM is released only after the last MMA has completed.
+// Every wait on an mbarrier is bounded.  No thread returns early: both CTAs meet
+// at the cluster barriers at start and end on every path, including after a
+// timeout, and the TMEM is released only after the last MMA has completed.  Those
+// barriers and the epilogue warps' named one (!FW) have no limit: after a failed
+// wait an epilogue warp goes on through its tiles, meeting the others once in each.
 #include "epilogue.cuh"
 #include "launch_util.h"
 #include "mxf4_rows.cuh"
@@ -92,7 +94,7 @@ constexpr int COLS_N = 256;              // epilogue column factors (BN used)
 constexpr uint16_t BOTH = 0x3;           // CTA mask of a commit to both ranks
 
 // Shared-memory layout per r^2 mode.  R2_EXACT needs 8 bytes of column
-// factors per column (epi::ColsF), R2_REFERENCE 16 (epi::ColsR); both leave
+// factors per column (epi::ColsF), R2_REFERENCE 16 (epi::ColsR2); both leave
 // room for six packed stages (more TMA lookahead than five: 2.576 -> 2.562
 // ms on the single region).
 template <int MODE>

@@ -7,11 +7,11 @@
 // the fused r^2 epilogue of qLD gemm_cpu.c:343-404); what differs is the
 // division of a small task.  The persistent kernel gives a task of up to one
 // tile per SM pair whole 256 x 240 tiles: most pairs stay idle, one pair
-// walks all K words, and eight of its twenty warps then run an epilogue that
-// nothing overlaps.  Measured, persistent against this kernel (us per launch
-// in a CUDA graph, SNPs x samples): single region 200 x 1,000 11.6 / 7.6,
-// 2,048 x 4,096 16.2 / 13.1, 64 x 50,000 72 / 19.7; two regions 731 x 530 x
-// 5,008 in reference mode 22.7 / 11.8.  A launch of one part per pair is bound
+// walks all K words, and eight of its warps then run an epilogue that nothing
+// overlaps.  Measured, persistent against this kernel (us per launch
+// in a CUDA graph, SNPs x samples): single region 200 x 1,000 8.0 / 5.9,
+// 2,048 x 4,096 12.1 / 11.3, 64 x 50,000 58 / 17.7; two regions 731 x 530 x
+// 5,008 in reference mode 17.0 / 10.4.  A launch of one part per pair is bound
 // by the latency of its steps: launch and setup, the first TMA, 0.235 us per
 // 256-sample stage (the handshakes; the MMAs take 0.12), the epilogue.  Here
 //   * the tile is 256 x bn with bn (16..240, a multiple of 16) chosen per
@@ -32,8 +32,10 @@
 // the MMAs, warps 2-17 workers, each thread up to two packed rows of every
 // fourth 256-sample stage.
 //
-// Every wait is bounded and no thread returns early: all CTAs of a cluster
-// meet at the cluster barriers on every path.
+// Every wait on an mbarrier is bounded and no thread returns early.  The named
+// barrier of the workers and the cluster barriers have no limit: every worker
+// warp meets the one once, and every warp of every CTA the others, on every path,
+// a failed wait included.
 #include <atomic>
 
 #include "epilogue.cuh"

@@ -221,18 +221,7 @@ __device__ __forceinline__ bool mbar_wait_acq_cluster(uint32_t bar, uint32_t par
     }
 }
 
-__device__ __forceinline__ void tc_mma_mxf4_pair(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                                 uint32_t idesc, uint32_t accumulate,
-                                                 uint32_t sfa, uint32_t sfb) {
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::2.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%6], p;\n\t}"
-        ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(sfa), "r"(sfb)
-        : "memory");
-}
-
-// The same with the descriptors as 32-bit halves: `alo` and `blo` hold a
+// One MMA of an SM pair, the descriptors as 32-bit halves: `alo` and `blo` hold a
 // sw128_desc's start address in 16-byte units (the other low bits are
 // constant, so a caller steps through its stages with one 32-bit add each)
 // and the high half is the same for every operand.
@@ -426,8 +415,8 @@ struct TileList {
         }
         return n;
     }
-    // decode() for a caller whose indices never decrease (a persistent CTA
-    // walking its tiles): the walk over B tiles resumes at (t, base), the B
+    // A and B tile of tile idx, for a caller whose indices never decrease (a
+    // persistent CTA walking its tiles): the walk over B tiles resumes at (t, base), the B
     // tile and the count of tiles before it where the previous call stopped,
     // so a call costs the B tiles stepped over instead of all of them.
     __host__ __device__ __forceinline__ void decode_from(int idx, int &ta, int &tb, int &t,
@@ -442,19 +431,6 @@ struct TileList {
                 return;
             }
             base += cc;
-        }
-        ta = tb = -1;
-    }
-    __host__ __device__ __forceinline__ void decode(int idx, int &ta, int &tb) const {
-        for (int t = 0; t < tiles_b; ++t) {
-            const int lo = ta_lo(tb0 + t);
-            const int c = ta_hi(tb0 + t) - lo;
-            if (c > 0 && idx < c) {
-                ta = lo + idx;
-                tb = tb0 + t;
-                return;
-            }
-            idx -= c > 0 ? c : 0;
         }
         ta = tb = -1;
     }
